@@ -42,9 +42,11 @@ struct DevBuf {
     }
 };
 
+// 16 bytes of slack: kernels read index arrays in aligned quads of 4 bytes,
+// whose last one may reach past the array (what lies there is not used).
 template <class T>
 inline T* upload(const std::vector<T>& h, DevBuf& b) {
-    b.ensure(h.size() * sizeof(T));
+    b.ensure(h.size() * sizeof(T) + 16);
     if (!h.empty()) GMR_CUDA(cudaMemcpy(b.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
     return static_cast<T*>(b.p);
 }

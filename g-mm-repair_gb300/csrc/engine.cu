@@ -210,7 +210,7 @@ __device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("gridd
 // [t0, t0 + gridDim.y) of Bt words each (blockIdx.y = tile).  Within a tile an
 // item is (unit, lane): G = Bt / VEC lanes per unit (rule, emission or row
 // segment), each lane moving VEC consecutive words.  G is a power of two
-// given as GLOG (shifts, no division); GLOG < 0 selects a generic G.
+// given as GLOG; GLOG < 0 selects a generic G (span_of).
 // The arena and the terminal table are tile-major ([tile][slot][Bt]) so the
 // values of one tile are dense; X and Y keep the caller's [row][Bw] layout.
 struct SweepArgs {
@@ -236,6 +236,10 @@ struct SweepArgs {
     const int32_t* rule_terms = nullptr;
     int64_t n_rule_terms = 0;
     int32_t cols = 0;
+    // Padded batch (Launch::padded): X has rows of x_words words at any
+    // alignment, read one word at a time by the prologue.  0: X is read in
+    // vectors like Y.
+    int x_words = 0;
 };
 
 struct LevelArgs {
@@ -268,20 +272,30 @@ struct LevelArgs {
     int level = 0;
 };
 
+// The units and the lane of one thread of block `block` of `blocks` (256
+// threads each): units u, u + stride, u + 2 stride, ... and one fixed lane, so
+// the loops over units hold no division.  A lane count that is no power of two
+// puts 256 / G whole units on a block and leaves the threads beyond them idle
+// (at G = 5 one of 256); above 256 lanes a block takes one unit and its
+// threads several lanes each (for_lanes).
+struct Span {
+    int64_t u, stride;
+    int lane;
+};
 template <int GLOG>
-__device__ __forceinline__ int64_t unit_of(int64_t t, int G) {
-    if constexpr (GLOG >= 0) return t >> GLOG;
-    else return t / G;
+__device__ __forceinline__ Span span_of(int G, int64_t block, int64_t blocks) {
+    if constexpr (GLOG >= 0) {
+        return {(block * 256 + threadIdx.x) >> GLOG, (blocks * 256) >> GLOG, (int)threadIdx.x & ((1 << GLOG) - 1)};
+    } else {
+        const int per = max(256 / G, 1), s = (int)threadIdx.x / G;
+        return {s < per ? block * per + s : (int64_t)1 << 40, blocks * per, (int)threadIdx.x - s * G};
+    }
 }
-template <int GLOG>
-__device__ __forceinline__ int lane_of(int64_t t, int G) {
-    if constexpr (GLOG >= 0) return (int)(t & ((1 << GLOG) - 1));
-    else return (int)(t % G);
-}
-template <int GLOG>
-__device__ __forceinline__ int64_t items_of(int64_t units, int G) {
-    if constexpr (GLOG >= 0) return units << GLOG;
-    else return units * G;
+template <int GLOG, class F>
+__device__ __forceinline__ void for_lanes(int G, const Span& sp, F&& f) {
+    if constexpr (GLOG >= 0) f(sp.lane);
+    else
+        for (int lane = sp.lane; lane < G; lane += 256) f(lane);
 }
 
 // Per-tile view of the value space: arena slots (refs >= 0) and terminals
@@ -352,40 +366,58 @@ __device__ __forceinline__ T* yptr(const SweepArgs& a, int64_t row, int tile, in
 
 // Prologue: Y = zero, T[0] = zero, T[q] = leaf(V[val], X[col]).
 template <class S, int VEC, int GLOG>
-__device__ __forceinline__ void do_prologue(const SweepArgs& a, int tile, int64_t t0, int64_t stride) {
+__device__ __forceinline__ void do_prologue(const SweepArgs& a, int tile, const Span& sp) {
     using T = typename S::T;
     const int64_t nq = a.rule_terms ? a.n_rule_terms : a.n_terms;
-    const int64_t ny = items_of<GLOG>(a.rows, a.G), nt = items_of<GLOG>(nq, a.G);
     T* Tt = static_cast<T*>(a.T) + (int64_t)tile * a.n_terms * a.Bt;
-    for (int64_t t = t0; t < ny + nt; t += stride) {
-        if (t < ny) {
-            vstore<T, VEC>(yptr<T>(a, unit_of<GLOG>(t, a.G), tile, lane_of<GLOG>(t, a.G), VEC), vzero<S, VEC>());
-        } else {
-            const int64_t u = t - ny;
-            const int64_t i = unit_of<GLOG>(u, a.G);
+    for_lanes<GLOG>(a.G, sp, [&](int lane) {
+        for (int64_t u = sp.u; u < a.rows + nq; u += sp.stride) {
+            if (u < a.rows) {
+                vstore<T, VEC>(yptr<T>(a, u, tile, lane, VEC), vzero<S, VEC>());
+                continue;
+            }
+            const int64_t i = u - a.rows;
             const int64_t q = a.rule_terms ? (int64_t)__ldg(a.rule_terms + i) : i;
-            const int lane = lane_of<GLOG>(u, a.G);
             Vec<T, VEC> out;
             if (q == 0) {
                 out = vzero<S, VEC>();
             } else {
                 float v = __ldg(a.V + __ldg(a.term_val + q - 1));
                 int32_t col = __ldg(a.term_col + q - 1);
-                Vec<T, VEC> x = vload<T, VEC>(static_cast<const T*>(a.X) + (int64_t)col * a.ldx +
-                                              (int64_t)tile * a.Bt + lane * VEC);
+                const int w0 = tile * a.Bt + lane * VEC;
+                const T* xp = static_cast<const T*>(a.X) + (int64_t)col * a.ldx + w0;
+                Vec<T, VEC> x;
+                if (a.x_words) {  // caller's rows of x_words words, any alignment: one word at a time
+#pragma unroll
+                    for (int j = 0; j < VEC; ++j) x.v[j] = w0 + j < a.x_words ? __ldg(xp + j) : S::zero();
+                } else {
+                    x = vload<T, VEC>(xp);
+                }
 #pragma unroll
                 for (int j = 0; j < VEC; ++j) out.v[j] = S::leaf(v, x.v[j]);
             }
             vstore<T, VEC>(Tt + q * a.Bt + lane * VEC, out);
         }
-    }
+    });
 }
 
 template <class S, int VEC, int GLOG>
 __global__ void __launch_bounds__(256) k_prologue(SweepArgs a) {
     dependents_may_launch();
-    do_prologue<S, VEC, GLOG>(a, a.t0 + blockIdx.y, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
-                              (int64_t)gridDim.x * blockDim.x);
+    do_prologue<S, VEC, GLOG>(a, a.t0 + blockIdx.y, span_of<GLOG>(a.G, blockIdx.x, gridDim.x));
+}
+
+// Rows of `from` words (stride ldi) copied to rows of ldo words: the padded
+// copy of X (the words past `from` are the semiring zero) and the caller's Y
+// from its padded copy (ldo = from: nothing to pad).
+template <class T>
+__global__ void __launch_bounds__(256) k_restride(const T* __restrict__ in, T* __restrict__ out, int64_t rows, int from,
+                                                  int ldi, int ldo, T pad) {
+    dependents_may_launch();
+    wait_for_previous_kernel();
+    const Span sp = span_of<-1>(ldo, blockIdx.x, gridDim.x);
+    for (int64_t r = sp.u; r < rows; r += sp.stride)
+        for (int w = sp.lane; w < ldo; w += 256) out[r * ldo + w] = w < from ? in[r * ldi + w] : pad;
 }
 
 // Push of two freshly computed values into the rows that emit them: the
@@ -411,51 +443,51 @@ __device__ __forceinline__ void push_rows(const SweepArgs& a, const LevelArgs& L
 // Evaluate the ops of one level, two items per thread in flight; with
 // L.pe_off set, each value is also pushed into its emitting rows of Y.
 template <class S, int VEC, int GLOG, bool CG = false, bool DIR = false>
-__device__ __forceinline__ void do_ops(const SweepArgs& a, const LevelArgs& L, int tile, int64_t t0,
-                                       int64_t stride) {
+__device__ __forceinline__ void do_ops(const SweepArgs& a, const LevelArgs& L, int tile, const Span& sp) {
     using T = typename S::T;
     const Values<S, VEC, CG> val(a, tile);
     T* out = static_cast<T*>(a.arena) + (int64_t)tile * a.n_ops * a.Bt;
-    const int64_t items = items_of<GLOG>(L.n_ops, a.G);
-    for (int64_t t = t0; t < items; t += 2 * stride) {
-        const int64_t tb = t + stride;
-        const bool hb = tb < items;
-        const int64_t sa = L.op_first + unit_of<GLOG>(t, a.G), sb = L.op_first + unit_of<GLOG>(hb ? tb : t, a.G);
-        const int la = lane_of<GLOG>(t, a.G), lb = lane_of<GLOG>(hb ? tb : t, a.G);
-        const int2 oa = __ldg(L.ops + sa), ob = __ldg(L.ops + sb);
-        Vec<T, VEC> la_v = val.template get_op<DIR>(oa.x, la), ra_v = val.template get_op<DIR>(oa.y, la);
-        Vec<T, VEC> lb_v = val.template get_op<DIR>(ob.x, lb), rb_v = val.template get_op<DIR>(ob.y, lb);
-        if (L.op_c) {
-            const float ca = __ldg(L.op_c + sa), cb = __ldg(L.op_c + sb);
+    for_lanes<GLOG>(a.G, sp, [&](int lane) {
+        // slots are below 2^31 (validate_plan), so 32-bit indices hold
+        const uint32_t first = (uint32_t)L.op_first, end = first + (uint32_t)L.n_ops, stride = (uint32_t)sp.stride;
+        if (sp.u >= L.n_ops) return;
+        for (uint32_t sa = first + (uint32_t)sp.u; sa < end; sa += 2 * stride) {
+            const bool hb = sa + stride < end;
+            const uint32_t sb = hb ? sa + stride : sa;
+            const int2 oa = __ldg(L.ops + sa), ob = __ldg(L.ops + sb);
+            Vec<T, VEC> la_v = val.template get_op<DIR>(oa.x, lane), ra_v = val.template get_op<DIR>(oa.y, lane);
+            Vec<T, VEC> lb_v = val.template get_op<DIR>(ob.x, lane), rb_v = val.template get_op<DIR>(ob.y, lane);
+            if (L.op_c) {
+                const float ca = __ldg(L.op_c + sa), cb = __ldg(L.op_c + sb);
 #pragma unroll
-            for (int j = 0; j < VEC; ++j) {
-                la_v.v[j] = S::apply(la_v.v[j], ca);
-                lb_v.v[j] = S::apply(lb_v.v[j], cb);
+                for (int j = 0; j < VEC; ++j) {
+                    la_v.v[j] = S::apply(la_v.v[j], ca);
+                    lb_v.v[j] = S::apply(lb_v.v[j], cb);
+                }
+            }
+            const Vec<T, VEC> va = voplus<S, VEC>(la_v, ra_v), vb = voplus<S, VEC>(lb_v, rb_v);
+            vstore<T, VEC>(out + (int64_t)sa * a.Bt + lane * VEC, va);
+            if (hb) vstore<T, VEC>(out + (int64_t)sb * a.Bt + lane * VEC, vb);
+            if (L.pe_off) {
+                push_rows<S, VEC>(a, L, sa, tile, lane, va);
+                if (hb) push_rows<S, VEC>(a, L, sb, tile, lane, vb);
             }
         }
-        const Vec<T, VEC> va = voplus<S, VEC>(la_v, ra_v), vb = voplus<S, VEC>(lb_v, rb_v);
-        vstore<T, VEC>(out + sa * a.Bt + la * VEC, va);
-        if (hb) vstore<T, VEC>(out + sb * a.Bt + lb * VEC, vb);
-        if (L.pe_off) {
-            push_rows<S, VEC>(a, L, sa, tile, la, va);
-            if (hb) push_rows<S, VEC>(a, L, sb, tile, lb, vb);
-        }
-    }
+    });
 }
 
 // One atomic per (emission, word): the reference's emit scheme.
 template <class S, int VEC, int GLOG, bool CG = false, bool DIR = false>
-__device__ __forceinline__ void do_emits_atomic(const SweepArgs& a, const LevelArgs& L, int tile, int64_t t0,
-                                                int64_t stride) {
+__device__ __forceinline__ void do_emits_atomic(const SweepArgs& a, const LevelArgs& L, int tile, const Span& sp) {
     using T = typename S::T;
     const Values<S, VEC, CG> val(a, tile);
-    const int64_t items = items_of<GLOG>(L.n_em, a.G);
-    for (int64_t t = t0; t < items; t += stride) {
-        const int64_t e = L.em_first + unit_of<GLOG>(t, a.G);
-        const int lane = lane_of<GLOG>(t, a.G);
-        const int32_t src = __ldg(L.em_src + e), row = __ldg(L.em_row + e);
-        vred<S, VEC>(yptr<T>(a, row, tile, lane, VEC), val.template get_em<DIR>(src, lane));
-    }
+    for_lanes<GLOG>(a.G, sp, [&](int lane) {
+        for (int64_t u = sp.u; u < L.n_em; u += sp.stride) {
+            const int64_t e = L.em_first + u;
+            const int32_t src = __ldg(L.em_src + e), row = __ldg(L.em_row + e);
+            vred<S, VEC>(yptr<T>(a, row, tile, lane, VEC), val.template get_em<DIR>(src, lane));
+        }
+    });
 }
 
 // Warp-segmented emits when G == 1: lane = emission; rows are sorted, so
@@ -489,13 +521,12 @@ __device__ __forceinline__ Vec<typename S::T, VEC> warp_segment_reduce(Vec<typen
 }
 
 template <class S, int VEC, bool CG = false, bool DIR = false>
-__device__ __forceinline__ void do_emits_warp(const SweepArgs& a, const LevelArgs& L, int tile, int64_t t0,
-                                              int64_t stride) {
+__device__ __forceinline__ void do_emits_warp(const SweepArgs& a, const LevelArgs& L, int tile, const Span& sp) {
     using T = typename S::T;
     const Values<S, VEC, CG> val(a, tile);
     const int lane = threadIdx.x & 31;
-    const int64_t n = L.n_em;
-    for (int64_t base = t0 - lane; base < n; base += 2 * stride) {  // warp-uniform trip count
+    const int64_t n = L.n_em, stride = sp.stride;  // one lane per unit: sp.u = this thread's emission
+    for (int64_t base = sp.u - lane; base < n; base += 2 * stride) {  // warp-uniform trip count
         const int64_t ea = base + lane, eb = base + stride + lane;
         const bool va = ea < n, vb = eb < n;
         const int32_t ra = va ? __ldg(L.em_row + L.em_first + ea) : -1 - lane;
@@ -512,57 +543,58 @@ __device__ __forceinline__ void do_emits_warp(const SweepArgs& a, const LevelArg
 }
 
 // Chunked segmented emits: each lane group walks em_chunk consecutive
-// emissions (loads four ahead), accumulating while the row stays the same.
+// emissions (a multiple of 4, aligned on the emission index), four values in
+// flight, accumulating while the row stays the same.
+//
+// Bound by the L1: a warp's load of values from as many lines as it has lane
+// groups takes that many tag cycles, and so does a load of row or source
+// indices, because the groups' chunks lie 64 bytes apart.  Indices are
+// therefore read four at a time (one 16-byte load instead of four 4-byte
+// ones): with single loads they took as many tag cycles as the values.
 template <class S, int VEC, int GLOG, bool CG = false, bool DIR = false>
-__device__ __forceinline__ void do_emits_chunk(const SweepArgs& a, const LevelArgs& L, int tile, int64_t t0,
-                                               int64_t stride) {
+__device__ __forceinline__ void do_emits_chunk(const SweepArgs& a, const LevelArgs& L, int tile, const Span& sp) {
     using T = typename S::T;
     const Values<S, VEC, CG> val(a, tile);
-    const int64_t groups = (L.n_em + L.em_chunk - 1) / L.em_chunk;
-    const int64_t items = items_of<GLOG>(groups, a.G);
-    const int32_t* rows = L.em_row + L.em_first;
-    const int32_t* srcs = L.em_src + L.em_first;
-    for (int64_t t = t0; t < items; t += stride) {
-        const int64_t g = unit_of<GLOG>(t, a.G);
-        const int lane = lane_of<GLOG>(t, a.G);
-        const int64_t e0 = g * L.em_chunk, e1 = min(e0 + (int64_t)L.em_chunk, L.n_em);
-        int32_t cur = __ldg(rows + e0);
-        Vec<T, VEC> acc = vzero<S, VEC>();
-        int64_t e = e0;
-        for (; e + 4 <= e1; e += 4) {
-            int32_t r[4], s[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                r[j] = __ldg(rows + e + j);
-                s[j] = __ldg(srcs + e + j);
-            }
-            Vec<T, VEC> v[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = val.template get_em<DIR>(s[j], lane);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (r[j] != cur) {
-                    vred<S, VEC>(yptr<T>(a, cur, tile, lane, VEC), acc);
-                    acc = v[j];
-                    cur = r[j];
-                } else {
-                    acc = voplus<S, VEC>(acc, v[j]);
+    const int skew = (int)(L.em_first & 3);  // emissions of the first quad that belong to the level below
+    const int64_t base = L.em_first - skew, n = L.n_em + skew;
+    const uint32_t groups = (uint32_t)((n + L.em_chunk - 1) / L.em_chunk);
+    for_lanes<GLOG>(a.G, sp, [&](int lane) {
+        if (sp.u >= groups) return;
+        for (uint32_t g = (uint32_t)sp.u; g < groups; g += (uint32_t)sp.stride) {
+            const int64_t at = (int64_t)g * L.em_chunk;
+            const int len = (int)min((int64_t)L.em_chunk, n - at), lo = g == 0 ? skew : 0;
+            int32_t cur = __ldg(L.em_row + base + at + lo);
+            Vec<T, VEC> acc = vzero<S, VEC>();
+            for (int q = 0; q < len; q += 4) {
+                int4 r = __ldg(reinterpret_cast<const int4*>(L.em_row + base + at + q));
+                int4 s = __ldg(reinterpret_cast<const int4*>(L.em_src + base + at + q));
+                if (q < lo || q + 4 > len) {  // a ragged end: the zero value there, and no change of row
+                    if (q < lo) r.x = cur, s.x = -1;
+                    if (q + 1 < lo) r.y = cur, s.y = -1;
+                    if (q + 2 < lo) r.z = cur, s.z = -1;
+                    if (q + 1 >= len) r.y = r.x, s.y = -1;
+                    if (q + 2 >= len) r.z = r.y, s.z = -1;
+                    if (q + 3 >= len) r.w = r.z, s.w = -1;
                 }
+                const Vec<T, VEC> v0 = val.template get_em<DIR>(s.x, lane), v1 = val.template get_em<DIR>(s.y, lane);
+                const Vec<T, VEC> v2 = val.template get_em<DIR>(s.z, lane), v3 = val.template get_em<DIR>(s.w, lane);
+                auto fold = [&](int32_t row, const Vec<T, VEC>& v) {
+                    if (row != cur) {
+                        vred<S, VEC>(yptr<T>(a, cur, tile, lane, VEC), acc);
+                        acc = v;
+                        cur = row;
+                    } else {
+                        acc = voplus<S, VEC>(acc, v);
+                    }
+                };
+                fold(r.x, v0);
+                fold(r.y, v1);
+                fold(r.z, v2);
+                fold(r.w, v3);
             }
+            vred<S, VEC>(yptr<T>(a, cur, tile, lane, VEC), acc);
         }
-        for (; e < e1; ++e) {
-            const int32_t r = __ldg(rows + e);
-            Vec<T, VEC> v = val.template get_em<DIR>(__ldg(srcs + e), lane);
-            if (r != cur) {
-                vred<S, VEC>(yptr<T>(a, cur, tile, lane, VEC), acc);
-                acc = v;
-                cur = r;
-            } else {
-                acc = voplus<S, VEC>(acc, v);
-            }
-        }
-        vred<S, VEC>(yptr<T>(a, cur, tile, lane, VEC), acc);
-    }
+    });
 }
 
 // Row-owned emits: one lane group folds a whole (level, row) segment and
@@ -570,14 +602,12 @@ __device__ __forceinline__ void do_emits_chunk(const SweepArgs& a, const LevelAr
 // (row, tile) belongs to exactly one segment and levels are separate launches,
 // so no atomics are needed and the (+,x) summation order is fixed.
 template <class S, int VEC, int GLOG, bool CG = false, bool DIR = false>
-__device__ __forceinline__ void do_emits_rows(const SweepArgs& a, const LevelArgs& L, int tile, int64_t t0,
-                                              int64_t stride) {
+__device__ __forceinline__ void do_emits_rows(const SweepArgs& a, const LevelArgs& L, int tile, const Span& sp) {
     using T = typename S::T;
     const Values<S, VEC, CG> val(a, tile);
-    const int64_t items = items_of<GLOG>(L.n_seg, a.G);
-    for (int64_t t = t0; t < items; t += stride) {
-        const int64_t s = L.seg_first + unit_of<GLOG>(t, a.G);
-        const int lane = lane_of<GLOG>(t, a.G);
+    for_lanes<GLOG>(a.G, sp, [&](int lane) {
+    for (int64_t u = sp.u; u < L.n_seg; u += sp.stride) {
+        const int64_t s = L.seg_first + u;
         const int64_t e0 = __ldg(L.seg_start + s), e1 = __ldg(L.seg_start + s + 1);
         const int32_t row = __ldg(L.seg_row + s);
         Vec<T, VEC> acc0 = vzero<S, VEC>(), acc1 = vzero<S, VEC>();
@@ -594,35 +624,36 @@ __device__ __forceinline__ void do_emits_rows(const SweepArgs& a, const LevelArg
         T* yp = yptr<T>(a, row, tile, lane, VEC);
         vstore<T, VEC>(yp, voplus<S, VEC>(vload_rw<T, VEC, CG>(yp), voplus<S, VEC>(acc0, acc1)));
     }
+    });
 }
 
 // Emission fold of one launch; DIR: the sources are terminal codes (see
 // SweepArgs::em_tcode).  A compile-time choice, so each fold keeps its batched
 // loads free of per-item branches.
 template <class S, int VEC, int GLOG, int EMIT, bool CG, bool DIR>
-__device__ __forceinline__ void emits_t(const SweepArgs& a, const LevelArgs& L, int tile, int64_t t0, int64_t stride) {
-    if constexpr (EMIT == GMR_EMIT_ATOMIC) do_emits_atomic<S, VEC, GLOG, CG, DIR>(a, L, tile, t0, stride);
-    else if constexpr (EMIT == GMR_EMIT_ROWS) do_emits_rows<S, VEC, GLOG, CG, DIR>(a, L, tile, t0, stride);
-    else if constexpr (GLOG == 0) do_emits_warp<S, VEC, CG, DIR>(a, L, tile, t0, stride);
-    else do_emits_chunk<S, VEC, GLOG, CG, DIR>(a, L, tile, t0, stride);
+__device__ __forceinline__ void emits_t(const SweepArgs& a, const LevelArgs& L, int tile, const Span& sp) {
+    if constexpr (EMIT == GMR_EMIT_ATOMIC) do_emits_atomic<S, VEC, GLOG, CG, DIR>(a, L, tile, sp);
+    else if constexpr (EMIT == GMR_EMIT_ROWS) do_emits_rows<S, VEC, GLOG, CG, DIR>(a, L, tile, sp);
+    else if constexpr (GLOG == 0) do_emits_warp<S, VEC, CG, DIR>(a, L, tile, sp);
+    else do_emits_chunk<S, VEC, GLOG, CG, DIR>(a, L, tile, sp);
 }
 
 // One level launch: blocks [0, em_blocks) fold emissions, the rest evaluate ops.
 // DIRK (direct terminals): 0 off; 1 rule children are terminal codes; 2 the
 // emissions too (the launch that folds the terminal emissions).
+// Resident blocks: 4 of 64 registers with 8-word lanes, 5 of 48 with 4-word
+// lanes (left alone the fold takes 59 and 4 blocks fit, which cost 10 % at
+// B = 64 and 128).
 template <class S, int VEC, int GLOG, int EMIT, int DIRK = 0>
-__global__ void __launch_bounds__(256, VEC == 8 ? 4 : 1) k_level(SweepArgs a, LevelArgs L) {
+__global__ void __launch_bounds__(256, VEC == 8 ? 4 : VEC == 4 ? 5 : 1) k_level(SweepArgs a, LevelArgs L) {
     dependents_may_launch();
     wait_for_previous_kernel();
     const int tile = a.t0 + blockIdx.y;
     if ((int)blockIdx.x < L.em_blocks) {
-        const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-        const int64_t stride = (int64_t)L.em_blocks * blockDim.x;
-        emits_t<S, VEC, GLOG, EMIT, false, DIRK == 2>(a, L, tile, t0, stride);
+        emits_t<S, VEC, GLOG, EMIT, false, DIRK == 2>(a, L, tile, span_of<GLOG>(a.G, blockIdx.x, L.em_blocks));
     } else {
-        const int64_t t0 = (int64_t)(blockIdx.x - L.em_blocks) * blockDim.x + threadIdx.x;
-        const int64_t stride = (int64_t)(gridDim.x - L.em_blocks) * blockDim.x;
-        do_ops<S, VEC, GLOG, false, DIRK >= 1>(a, L, tile, t0, stride);
+        do_ops<S, VEC, GLOG, false, DIRK >= 1>(
+            a, L, tile, span_of<GLOG>(a.G, (int)blockIdx.x - L.em_blocks, (int)gridDim.x - L.em_blocks));
     }
 }
 
@@ -652,8 +683,7 @@ __global__ void __launch_bounds__(256, VEC == 8 ? 4 : 1) k_level_staged(SweepArg
     wait_for_previous_kernel();
     const int tile = a.t0 + blockIdx.y;
     if ((int)blockIdx.x < L.em_blocks) {
-        emits_t<S, VEC, GLOG, GMR_EMIT_SEGMENTED, false, false>(
-            a, L, tile, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)L.em_blocks * blockDim.x);
+        emits_t<S, VEC, GLOG, GMR_EMIT_SEGMENTED, false, false>(a, L, tile, span_of<GLOG>(a.G, blockIdx.x, L.em_blocks));
         return;
     }
     constexpr int kUnits = 256 >> GLOG;  // rules per pass of the block
@@ -796,9 +826,8 @@ __device__ __forceinline__ bool grid_barrier(const PersistArgs& P, int phase) {
 
 template <class S, int VEC, int GLOG, int EMIT>
 __global__ void __launch_bounds__(256) k_persistent(SweepArgs a, LevelArgs L0, PersistArgs P) {
-    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    do_prologue<S, VEC, GLOG>(a, 0, t0, stride);
+    const Span sp = span_of<GLOG>(a.G, blockIdx.x, gridDim.x);
+    do_prologue<S, VEC, GLOG>(a, 0, sp);
     if (!grid_barrier(P, 0)) return;
     for (int k = 1; k <= P.depth + 1; ++k) {
         LevelArgs L = L0;
@@ -812,8 +841,8 @@ __global__ void __launch_bounds__(256) k_persistent(SweepArgs a, LevelArgs L0, P
         L.n_em = P.em_off[k] - P.em_off[k - 1];
         L.seg_first = P.seg_off[k - 1];
         L.n_seg = P.seg_off[k] - P.seg_off[k - 1];
-        emits_t<S, VEC, GLOG, EMIT, true, false>(a, L, 0, t0, stride);
-        do_ops<S, VEC, GLOG, true, false>(a, L, 0, t0, stride);
+        emits_t<S, VEC, GLOG, EMIT, true, false>(a, L, 0, sp);
+        do_ops<S, VEC, GLOG, true, false>(a, L, 0, sp);
         if (!grid_barrier(P, k)) return;
     }
 }
@@ -838,10 +867,11 @@ struct PackGrammar {
 // The grammar's argument structs are copied into locals first: read through
 // a pointer they would be reloaded from global memory inside the loops.
 template <class S, int VEC, int GLOG, int EMIT>
-__device__ __forceinline__ void pack_phase(const PackGrammar& g, int k, int64_t t0, int64_t stride) {
+__device__ __forceinline__ void pack_phase(const PackGrammar& g, int k) {
     const SweepArgs a = g.a;
+    const Span sp = span_of<GLOG>(a.G, blockIdx.x, gridDim.x);
     if (k == 0) {
-        do_prologue<S, VEC, GLOG>(a, 0, t0, stride);
+        do_prologue<S, VEC, GLOG>(a, 0, sp);
         return;
     }
     LevelArgs L = g.L;
@@ -855,30 +885,28 @@ __device__ __forceinline__ void pack_phase(const PackGrammar& g, int k, int64_t 
     L.n_em = g.em_off[k] - g.em_off[k - 1];
     L.seg_first = g.seg_off[k - 1];
     L.n_seg = g.seg_off[k] - g.seg_off[k - 1];
-    emits_t<S, VEC, GLOG, EMIT, true, false>(a, L, 0, t0, stride);
-    do_ops<S, VEC, GLOG, true, false>(a, L, 0, t0, stride);
+    emits_t<S, VEC, GLOG, EMIT, true, false>(a, L, 0, sp);
+    do_ops<S, VEC, GLOG, true, false>(a, L, 0, sp);
 }
 
 template <class S, int EMIT>
 __global__ void __launch_bounds__(256) k_pack(const PackGrammar* __restrict__ gs, int n, int max_depth, PersistArgs P) {
-    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int k = 0; k <= max_depth + 1; ++k) {
         for (int i = 0; i < n; ++i) {
             const PackGrammar& g = gs[i];
             if (k > g.depth + 1) continue;
             switch (g.kind) {
-                case 0: pack_phase<S, 4, 0, EMIT>(g, k, t0, stride); break;
-                case 1: pack_phase<S, 4, 1, EMIT>(g, k, t0, stride); break;
-                case 2: pack_phase<S, 4, 2, EMIT>(g, k, t0, stride); break;
-                case 3: pack_phase<S, 4, 3, EMIT>(g, k, t0, stride); break;
-                case 4: pack_phase<S, 4, 4, EMIT>(g, k, t0, stride); break;
-                case 5: pack_phase<S, 4, 5, EMIT>(g, k, t0, stride); break;
-                case 6: pack_phase<S, 4, -1, EMIT>(g, k, t0, stride); break;
-                case 7: pack_phase<S, 2, 0, EMIT>(g, k, t0, stride); break;
-                case 8: pack_phase<S, 1, 0, EMIT>(g, k, t0, stride); break;
-                case 9: pack_phase<S, 2, -1, EMIT>(g, k, t0, stride); break;
-                default: pack_phase<S, 1, -1, EMIT>(g, k, t0, stride); break;
+                case 0: pack_phase<S, 4, 0, EMIT>(g, k); break;
+                case 1: pack_phase<S, 4, 1, EMIT>(g, k); break;
+                case 2: pack_phase<S, 4, 2, EMIT>(g, k); break;
+                case 3: pack_phase<S, 4, 3, EMIT>(g, k); break;
+                case 4: pack_phase<S, 4, 4, EMIT>(g, k); break;
+                case 5: pack_phase<S, 4, 5, EMIT>(g, k); break;
+                case 6: pack_phase<S, 4, -1, EMIT>(g, k); break;
+                case 7: pack_phase<S, 2, 0, EMIT>(g, k); break;
+                case 8: pack_phase<S, 1, 0, EMIT>(g, k); break;
+                case 9: pack_phase<S, 2, -1, EMIT>(g, k); break;
+                default: pack_phase<S, 1, -1, EMIT>(g, k); break;
             }
         }
         if (!grid_barrier(P, k)) return;
@@ -899,10 +927,9 @@ struct PackLaunch {
 
 template <class S, int VEC, int GLOG, int EMIT>
 __device__ __forceinline__ void pack_level_part(const PackGrammar& g, int k, int b, int nb, int eb) {
-    const int64_t tid = threadIdx.x;
     const SweepArgs a = g.a;
     if (k == 0) {
-        do_prologue<S, VEC, GLOG>(a, 0, (int64_t)b * blockDim.x + tid, (int64_t)nb * blockDim.x);
+        do_prologue<S, VEC, GLOG>(a, 0, span_of<GLOG>(a.G, b, nb));
         return;
     }
     LevelArgs L = g.L;
@@ -916,8 +943,8 @@ __device__ __forceinline__ void pack_level_part(const PackGrammar& g, int k, int
     L.n_em = g.em_off[k] - g.em_off[k - 1];
     L.seg_first = g.seg_off[k - 1];
     L.n_seg = g.seg_off[k] - g.seg_off[k - 1];
-    if (b < eb) emits_t<S, VEC, GLOG, EMIT, false, false>(a, L, 0, (int64_t)b * blockDim.x + tid, (int64_t)eb * blockDim.x);
-    else do_ops<S, VEC, GLOG, false, false>(a, L, 0, (int64_t)(b - eb) * blockDim.x + tid, (int64_t)(nb - eb) * blockDim.x);
+    if (b < eb) emits_t<S, VEC, GLOG, EMIT, false, false>(a, L, 0, span_of<GLOG>(a.G, b, eb));
+    else do_ops<S, VEC, GLOG, false, false>(a, L, 0, span_of<GLOG>(a.G, b - eb, nb - eb));
 }
 
 template <class S, int EMIT>
@@ -962,12 +989,15 @@ static constexpr int64_t kChunkSlots = 1 << 19;  // source slots per chunk (64 M
 struct Launch {
     int semiring, B, Bw, VEC, G, variant, emit, chunk;
     int Bt, ntile, tile_levels;
+    int Bp;       // words per value inside the engine: Bw, or more when padded
+    bool padded;  // X and Y rows of Bw words go through padded copies (resolve_launch)
     int push_mode;  // GMR_PUSH_*
     unsigned long long spin_limit;
     std::vector<uint8_t> lv;  // per-launch variant (index = launch slot), empty = uniform emit/chunk
     bool operator==(const Launch& o) const {
         return semiring == o.semiring && B == o.B && Bw == o.Bw && VEC == o.VEC && variant == o.variant &&
-               emit == o.emit && chunk == o.chunk && Bt == o.Bt && tile_levels == o.tile_levels &&
+               emit == o.emit && chunk == o.chunk && Bt == o.Bt && Bp == o.Bp && padded == o.padded &&
+               tile_levels == o.tile_levels &&
                push_mode == o.push_mode && lv == o.lv;
     }
 };
@@ -991,6 +1021,7 @@ struct gmr_engine {
     std::vector<int64_t> lvl_off, em_off, seg_off;
     gmr::DevBuf ops, op_c, em_src, em_row, seg_row, seg_start, term_val, term_col, V;
     gmr::DevBuf arena, T, hX, hY;  // scratch
+    gmr::DevBuf padX, padY;        // scratch: X and Y in padded rows (Launch::padded)
     gmr::DevBuf hX2, hY2;          // second staging pair of the pipelined host-buffer multiply
     cudaStream_t copy_in = nullptr, copy_out = nullptr;
     cudaEvent_t pipe_ev[6] = {};    // per staging slot: X copied in, multiply done, Y copied out
@@ -1166,7 +1197,8 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
     SweepArgs a;
     a.arena = e->arena.p;
     a.T = e->T.p;
-    a.Y = Y;
+    using T = typename S::T;
+    a.Y = lc.padded ? e->padY.p : Y;
     a.X = X;
     a.V = static_cast<const float*>(e->V.p);
     a.term_val = static_cast<const int32_t*>(e->term_val.p);
@@ -1175,7 +1207,7 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
     a.n_ops = e->n_ops;
     a.rows = e->rows;
     a.ldx = lc.Bw;
-    a.ldy = lc.Bw;
+    a.ldy = lc.Bp;
     a.Bt = lc.Bt;
     a.G = lc.G;
     a.t0 = 0;
@@ -1194,6 +1226,15 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
         ++launches;
         if (t_timer && mark) t_timer->mark();
     };
+    if (lc.padded && e->direct_terms) {  // every launch gathers X: give it aligned rows
+        launch_kernel(k_restride<T>, dim3(blocks_for((int64_t)e->cols * lc.Bp, 1)), 0, st, false, static_cast<const T*>(X),
+                      static_cast<T*>(e->padX.p), (int64_t)e->cols, lc.Bw, lc.Bw, lc.Bp, T(0));
+        after(false);
+        a.X = e->padX.p;
+        a.ldx = lc.Bp;
+    } else if (lc.padded) {
+        a.x_words = lc.Bw;
+    }
     {
         int64_t items = (e->rows + (e->direct_terms ? e->n_rule_terms : e->n_terms)) * (int64_t)lc.G;
         dim3 grid(blocks_for(items, lc.ntile), lc.ntile);
@@ -1247,6 +1288,7 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
             by_chunk = false;
         }
         if (chunk <= 0) chunk = 16;
+        chunk = (chunk + 3) & ~3;  // the fold reads its indices four at a time
         L.em_chunk = chunk;
         int64_t nops = 0, nem = 0, nseg = 0;
         if (k_ops >= 1) {
@@ -1367,7 +1409,12 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
                 else level(k, k, 0, lc.ntile, false, lo, hi, c - 1 < nec ? e->ch_off[k] + c - 1 : -2, c == n_oc - 1);
             }
         }
-        level(0, D, 0, lc.ntile, false);
+        level(0, D, 0, lc.ntile, false, -1, -1, -1, !lc.padded);
+    }
+    if (lc.padded) {
+        launch_kernel(k_restride<T>, dim3(blocks_for((int64_t)e->rows * lc.Bw, 1)), 0, st, pdl,
+                      static_cast<const T*>(e->padY.p), static_cast<T*>(Y), (int64_t)e->rows, lc.Bw, lc.Bp, lc.Bw, T(0));
+        after();
     }
     if (staged) GMR_CUDA(cudaMemcpyAsync(e->status_host, e->stage_err(), 8, cudaMemcpyDeviceToHost, st));
     GMR_CUDA(cudaGetLastError());
@@ -1416,7 +1463,7 @@ static void launch_persistent_t(gmr_engine* e, const Launch& lc, const void* X, 
     L.em_row = static_cast<const int32_t*>(e->em_row.p);
     L.seg_row = static_cast<const int32_t*>(e->seg_row.p);
     L.seg_start = static_cast<const int64_t*>(e->seg_start.p);
-    L.em_chunk = lc.chunk > 0 ? lc.chunk : 16;
+    L.em_chunk = lc.chunk > 0 ? (lc.chunk + 3) & ~3 : 16;
     PersistArgs P;
     P.lvl_off = static_cast<const int64_t*>(e->d_lvl_off.p);
     P.em_off = static_cast<const int64_t*>(e->d_em_off.p);
@@ -1493,7 +1540,9 @@ static void launch_chain_s(gmr_engine* e, const Launch& lc, const void* X, void*
                 case 2: return launch_chain_t<S, 8, 1>(e, lc, X, Y, st, n);
                 case 4: return launch_chain_t<S, 8, 2>(e, lc, X, Y, st, n);
                 case 8: return launch_chain_t<S, 8, 3>(e, lc, X, Y, st, n);
-                default: return launch_chain_t<S, 8, 4>(e, lc, X, Y, st, n);
+                case 16: return launch_chain_t<S, 8, 4>(e, lc, X, Y, st, n);
+                default:
+                    if constexpr (std::is_same<S, SPlus>::value) return launch_chain_t<S, 8, -1>(e, lc, X, Y, st, n);
             }
         }
     }
@@ -1518,8 +1567,25 @@ static int auto_tile(gmr_engine*, int Bw) {
     return bt;
 }
 
-// max_vec: the widest lane access a caller's kernels instantiate (the pack
-// and the left product stop at 4 words).
+// max_vec: the widest lane access a caller's kernels instantiate (the pack's
+// single-kernel modes stop at 4 words and take X and Y as they are).
+//
+// Padded batches.  Rows of X and Y that 16-byte accesses cannot reach (an odd
+// batch width, a pointer that is not 16-byte aligned) used to drop the whole
+// sweep to 4-byte lanes, a quarter of the bytes a load could bring.  The
+// values inside the engine are its own, so they are laid out in Bp words per
+// value, a multiple of 8 (whole 32-byte sectors; of 4 up to 4 words): the
+// prologue reads X a word at a time (once per terminal), the folds update a
+// padded Y with vector reductions, and a last kernel copies Y's rows to the
+// caller.  Batches beyond 128 words become tiles of at most 128.  1 to 3 words
+// keep their layout: there a value is one sector either way.  Rows that 16-byte
+// accesses do reach are padded too where the wider value measured faster: 12
+// words (16: a power of two of lanes), and (+,x) from 28 words, where 8-word
+// lanes need multiples of 8 (36 / 60 / 100 words: 14.0 / 12.2 / 11.6 us a word
+// unpadded, 40 / 64 / 104: 11.6 / 8.7 / 9.7); (min,+) stays on 4-word lanes,
+// where 36 -> 40 words measured slower.  One multiply, before -> now:
+// 30,001 x 3,001, B = 33: 820 -> 355 us; 50,000 x 5,000: B = 5 287 -> 208 us,
+// B = 7 336 -> 207 us, B = 33 1019 -> 471 us, B = 129 3620 -> 1397 us.
 static Launch resolve_launch(gmr_engine* e, int semiring, int B, const void* X, void* Y, const gmr_config* cfg,
                              int max_vec = 8) {
     Launch lc{};
@@ -1541,30 +1607,41 @@ static Launch resolve_launch(gmr_engine* e, int semiring, int B, const void* X, 
     lc.push_mode = cfg ? cfg->push : GMR_PUSH_AUTO;
     if (lc.push_mode < GMR_PUSH_AUTO || lc.push_mode > GMR_PUSH_INTERLEAVE) throw Error(GMR_ERR_ARG, "unknown push mode");
     lc.chunk = cfg && cfg->ops_per_cta > 0 ? cfg->ops_per_cta : 16;
-    int bt = cfg && cfg->vec_tile > 0 ? cfg->vec_tile : auto_tile(e, lc.Bw);
-    if (bt > lc.Bw || lc.Bw % bt != 0) bt = lc.Bw;  // tiles must divide the batch
+    auto aligned = [&](size_t al) { return ((uintptr_t)X % al == 0) && ((uintptr_t)Y % al == 0); };
+    const bool tile_asked = cfg && cfg->vec_tile > 0 && cfg->vec_tile <= lc.Bw && lc.Bw % cfg->vec_tile == 0;
+    int bt = tile_asked ? cfg->vec_tile : cfg && cfg->vec_tile > 0 ? lc.Bw : auto_tile(e, lc.Bw);  // tiles must divide the batch
     if (lc.variant == GMR_VARIANT_PERSISTENT) bt = lc.Bw;  // one tile: the whole batch in one launch
+    lc.Bp = lc.Bw;
+    lc.padded = max_vec >= 8 && lc.variant != GMR_VARIANT_PERSISTENT && !tile_asked &&
+                ((lc.Bw >= 4 && (lc.Bw % 4 != 0 || !aligned(16))) ||
+                 (lc.Bw % 8 != 0 && (lc.Bw == 12 || (semiring == GMR_PLUS_TIMES && lc.Bw >= 28))));
+    if (lc.padded) {
+        const int nt = (lc.Bw + 127) / 128, per = (lc.Bw + nt - 1) / nt;
+        bt = per <= 4 ? 4 : (per + 7) / 8 * 8;
+        lc.Bp = bt * nt;
+    }
     lc.Bt = bt;
-    lc.ntile = lc.Bw / bt;
+    lc.ntile = lc.Bp / bt;
     lc.tile_levels = cfg && cfg->tile_levels > 0 ? cfg->tile_levels : e->depth;
     if (!cfg || cfg->tile_levels <= 0) {
         // tile the levels whose values overflow the budget at full width
         int K = 0;
         for (int k = 1; k <= e->depth; ++k)
-            if ((e->lvl_off[k] - e->lvl_off[k - 1]) * (int64_t)lc.Bw * 4 > (16ll << 20)) K = k;
+            if ((e->lvl_off[k] - e->lvl_off[k - 1]) * (int64_t)lc.Bp * 4 > (16ll << 20)) K = k;
         lc.tile_levels = std::max(K, 1);
     }
-    auto aligned = [&](size_t al) { return ((uintptr_t)X % al == 0) && ((uintptr_t)Y % al == 0); };
     int lane_bytes = cfg && cfg->lane_bytes ? cfg->lane_bytes : e->lane_bytes;
     if (lane_bytes != 0 && lane_bytes != 16 && lane_bytes != 32) throw Error(GMR_ERR_ARG, "lane_bytes must be 0, 16 or 32");
-    // 8 words per lane: fp32 / int32 tiles of 8..128 words (powers of two), 32-byte aligned X and Y
-    const bool v8_ok = max_vec >= 8 && semiring != GMR_BOOLEAN && lc.Bt % 8 == 0 && lc.Bw % 8 == 0 &&
-                       lc.Bt <= 128 && (lc.Bt & (lc.Bt - 1)) == 0 && aligned(32);
+    // 8 words per lane: fp32 / int32 tiles of 8..128 words (int32: powers of two), 32-byte aligned X and Y
+    const bool pow2 = (lc.Bt & (lc.Bt - 1)) == 0;
+    const bool v8_ok = max_vec >= 8 && semiring != GMR_BOOLEAN && lc.Bt % 8 == 0 && lc.Bp % 8 == 0 && lc.Bt <= 128 &&
+                       (pow2 || (semiring == GMR_PLUS_TIMES && lc.variant != GMR_VARIANT_PERSISTENT)) &&
+                       (lc.padded || aligned(32));
     // measured on the 200k x 10k grammar: 32-byte lanes win for (+,x) tiles of
     // >= 32 words (B = 32 / 64 / 128), lose at 8 words and for (min,+)
     if (lane_bytes == 0) lane_bytes = semiring == GMR_PLUS_TIMES && lc.Bt >= 32 ? 32 : 16;
     if (lane_bytes == 32 && v8_ok) lc.VEC = 8;
-    else if (lc.Bt % 4 == 0 && lc.Bw % 4 == 0 && aligned(16)) lc.VEC = 4;
+    else if (lc.Bt % 4 == 0 && lc.Bp % 4 == 0 && (lc.padded || aligned(16))) lc.VEC = 4;
     else if (lc.Bt % 2 == 0 && lc.Bw % 2 == 0 && aligned(8)) lc.VEC = 2;
     else lc.VEC = 1;
     lc.G = lc.Bt / lc.VEC;
@@ -1573,16 +1650,20 @@ static Launch resolve_launch(gmr_engine* e, int semiring, int B, const void* X, 
 
 // Grows the value arena and terminal table; cached graphs bake these
 // addresses in, so any reallocation drops them (after the device is idle).
-static void ensure_scratch(gmr_engine* e, int Bw) {
-    const size_t na = (size_t)std::max<int64_t>(e->n_ops, 1) * Bw * 4;
-    const size_t nt = (size_t)std::max<int64_t>(e->n_terms, 1) * Bw * 4;
-    if (na <= e->arena.bytes && nt <= e->T.bytes) return;
+static void ensure_scratch(gmr_engine* e, int words, bool padded = false) {
+    const size_t na = (size_t)std::max<int64_t>(e->n_ops, 1) * words * 4;
+    const size_t nt = (size_t)std::max<int64_t>(e->n_terms, 1) * words * 4;
+    const size_t ny = padded ? (size_t)e->rows * words * 4 : 0;
+    const size_t nx = padded && e->direct_terms ? (size_t)e->cols * words * 4 : 0;
+    if (na <= e->arena.bytes && nt <= e->T.bytes && ny <= e->padY.bytes && nx <= e->padX.bytes) return;
     GMR_CUDA(cudaDeviceSynchronize());
     for (auto& g : e->graphs)
         if (g.exec) cudaGraphExecDestroy(g.exec);
     e->graphs.clear();
     e->arena.ensure(na);
     e->T.ensure(nt);
+    e->padY.ensure(ny);
+    e->padX.ensure(nx);
 }
 
 static void multiply_device(gmr_engine* e, int semiring, const void* X, void* Y, int B, const gmr_config* cfg,
@@ -1593,7 +1674,7 @@ static void multiply_device(gmr_engine* e, int semiring, const void* X, void* Y,
     if (((uintptr_t)X | (uintptr_t)Y) % 4 != 0) throw Error(GMR_ERR_ARG, "X and Y must be 4-byte aligned");
     Launch lc = resolve_launch(e, semiring, B, X, Y, cfg);
     if (eager && lc.variant == GMR_VARIANT_GRAPH) lc.variant = GMR_VARIANT_FUSED;
-    ensure_scratch(e, lc.Bw);
+    ensure_scratch(e, lc.Bp, lc.padded);
     int64_t launches = 0;
     if (lc.variant == GMR_VARIANT_GRAPH) {
         GraphEntry* hit = nullptr;
@@ -2186,7 +2267,7 @@ extern "C" int64_t gmr_engine_device_bytes(const gmr_engine* e) {
     if (!e) return -1;
     int64_t t = 0;
     auto bufs = const_cast<gmr_engine*>(e)->schedule_bufs();
-    for (auto* b : {&e->arena, &e->T, &e->hX, &e->hY}) bufs.push_back(const_cast<DevBuf*>(b));
+    for (auto* b : {&e->arena, &e->T, &e->padX, &e->padY, &e->hX, &e->hY}) bufs.push_back(const_cast<DevBuf*>(b));
     for (auto* b : bufs) t += (int64_t)b->bytes;
     return t;
 }
@@ -2200,7 +2281,7 @@ extern "C" void gmr_engine_free(gmr_engine* e) {
         for (auto& g : e->graphs)
             if (g.exec) cudaGraphExecDestroy(g.exec);
         for (auto* b : e->schedule_bufs()) b->release();
-        for (auto* b : {&e->arena, &e->T, &e->hX, &e->hY, &e->hX2, &e->hY2}) b->release();
+        for (auto* b : {&e->arena, &e->T, &e->padX, &e->padY, &e->hX, &e->hY, &e->hX2, &e->hY2}) b->release();
         for (auto ev : e->pipe_ev)
             if (ev) cudaEventDestroy(ev);
         for (auto s2 : {e->copy_in, e->copy_out})
@@ -2273,25 +2354,25 @@ __device__ __forceinline__ void left_flush(const LeftArgs& a, int32_t u, int lan
 template <class S, int VEC, int GLOG>
 __global__ void __launch_bounds__(256) k_left_zero(LeftArgs a) {
     using T = typename S::T;
-    const int64_t items = items_of<GLOG>(a.count, a.G);  // count = straddling targets
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < items; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t u = __ldg(a.split + unit_of<GLOG>(t, a.G));
-        const int lane = lane_of<GLOG>(t, a.G);
+    const Span sp = span_of<GLOG>(a.G, blockIdx.x, gridDim.x);
+    for_lanes<GLOG>(a.G, sp, [&](int lane) {
+    for (int64_t i = sp.u; i < a.count; i += sp.stride) {  // count = straddling targets
+        const int64_t u = __ldg(a.split + i);
         T* p = u < a.n_ops ? static_cast<T*>(a.down) + u * a.Bw : static_cast<T*>(a.tdown) + (u - a.n_ops) * a.Bw;
         vstore<T, VEC>(p + lane * VEC, vzero<S, VEC>());
     }
+    });
 }
 
 template <class S, int VEC, int GLOG>
 __global__ void __launch_bounds__(256) k_left_fold(LeftArgs a) {
     using T = typename S::T;
     const int64_t groups = (a.count + kLeftChunk - 1) / kLeftChunk;
-    const int64_t items = items_of<GLOG>(groups, a.G);
     const int32_t* src = a.src + a.first;
     const int32_t* tgt = a.tgt + a.first;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < items; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t g = unit_of<GLOG>(t, a.G);
-        const int lane = lane_of<GLOG>(t, a.G);
+    const Span sp = span_of<GLOG>(a.G, blockIdx.x, gridDim.x);
+    for_lanes<GLOG>(a.G, sp, [&](int lane) {
+    for (int64_t g = sp.u; g < groups; g += sp.stride) {
         const int64_t e0 = g * kLeftChunk, e1 = min(e0 + kLeftChunk, a.count);
         int32_t cur = __ldg(tgt + e0);
         bool whole = e0 == 0 || __ldg(tgt + e0 - 1) != cur;  // cur's first edge is in this chunk
@@ -2334,16 +2415,16 @@ __global__ void __launch_bounds__(256) k_left_fold(LeftArgs a) {
         const bool ends = e1 == a.count || __ldg(tgt + e1) != cur;  // cur's last edge is in this chunk
         left_flush<S, VEC>(a, cur, lane, whole && ends, acc);
     }
+    });
 }
 
 template <class S, int VEC, int GLOG>
 __global__ void __launch_bounds__(256) k_left_columns(LeftArgs a) {
     using T = typename S::T;
-    const int64_t items = items_of<GLOG>(a.count, a.G);  // count = cols
     const T* tdown = static_cast<const T*>(a.tdown);
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < items; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t c = unit_of<GLOG>(t, a.G);
-        const int lane = lane_of<GLOG>(t, a.G);
+    const Span sp = span_of<GLOG>(a.G, blockIdx.x, gridDim.x);
+    for_lanes<GLOG>(a.G, sp, [&](int lane) {
+    for (int64_t c = sp.u; c < a.count; c += sp.stride) {  // count = cols
         Vec<T, VEC> acc = vzero<S, VEC>();
         for (int64_t i = __ldg(a.tcol_off + c), i1 = __ldg(a.tcol_off + c + 1); i < i1; ++i) {
             const int32_t q = __ldg(a.tcol_q + i);
@@ -2356,6 +2437,7 @@ __global__ void __launch_bounds__(256) k_left_columns(LeftArgs a) {
         }
         vstore<T, VEC>(static_cast<T*>(a.Y) + c * a.Bw + lane * VEC, acc);
     }
+    });
 }
 
 template <class S, int VEC, int GLOG>
@@ -2579,7 +2661,7 @@ extern "C" int gmr_engine_fixpoint(gmr_engine* e, int semiring, void* dX, void* 
         if (max_iters == 0) return;
         Launch lc = resolve_launch(e, semiring, B, dX, dY, nullptr);
         if (lc.variant == GMR_VARIANT_GRAPH || lc.variant == GMR_VARIANT_PERSISTENT) lc.variant = GMR_VARIANT_FUSED;
-        ensure_scratch(e, lc.Bw);
+        ensure_scratch(e, lc.Bp, lc.padded);
         const int64_t n = (int64_t)e->rows * lc.Bw;
         e->sync.ensure(64);
         int* flag = reinterpret_cast<int*>(static_cast<unsigned char*>(e->sync.p) + 8);
@@ -2615,7 +2697,7 @@ struct gmr_pack {
     cudaGraphExec_t exec = nullptr;
     std::vector<gmr::Launch> key_lc;
     std::vector<const void*> key_x;
-    std::vector<void*> key_y, key_arena;
+    std::vector<void*> key_y, key_scratch;  // key_scratch: every engine's scratch buffers (scratch_of)
     int64_t launches = 0;
     int device = 0;
     // one persistent launch (GMR_PACK_PERSISTENT): grammar table on the
@@ -2632,6 +2714,14 @@ struct gmr_pack {
 };
 
 namespace gmr {
+
+// The scratch addresses a captured chain of these engines bakes in.
+static std::vector<void*> scratch_of(const std::vector<gmr_engine*>& engines) {
+    std::vector<void*> p;
+    for (auto* e : engines)
+        for (auto* b : {&e->arena, &e->T, &e->padX, &e->padY}) p.push_back(b->p);
+    return p;
+}
 
 static int pack_kind(const Launch& lc) {
     if (lc.VEC == 4) {
@@ -2868,7 +2958,7 @@ extern "C" int gmr_pack_multiply(gmr_pack* p, const int* semirings, const void* 
             if (B[i] < 1) throw Error(GMR_ERR_ARG, "B must be >= 1");
             if (((uintptr_t)dX[i] | (uintptr_t)dY[i]) % 4 != 0) throw Error(GMR_ERR_ARG, "misaligned X or Y");
             Launch lc = resolve_launch(e, semirings[i], B[i], dX[i], dY[i], nullptr, one_kernel ? 4 : 8);
-            ensure_scratch(e, lc.Bw);
+            ensure_scratch(e, lc.Bp, lc.padded);
             lcs.push_back(lc);
         }
         p->last_persistent = false;
@@ -2880,10 +2970,9 @@ extern "C" int gmr_pack_multiply(gmr_pack* p, const int* semirings, const void* 
             pack_levels(p, semirings[0], lcs, dX, dY, static_cast<cudaStream_t>(stream));
             return;
         }
-        bool hit = p->exec != nullptr && p->key_lc.size() == (size_t)n;
+        bool hit = p->exec != nullptr && p->key_lc.size() == (size_t)n && p->key_scratch == scratch_of(p->engines);
         for (int i = 0; hit && i < n; ++i)
-            hit = p->key_lc[i] == lcs[i] && p->key_x[i] == dX[i] && p->key_y[i] == dY[i] &&
-                  p->key_arena[i] == p->engines[i]->arena.p;
+            hit = p->key_lc[i] == lcs[i] && p->key_x[i] == dX[i] && p->key_y[i] == dY[i];
         if (!hit) {
             if (p->exec) cudaGraphExecDestroy(p->exec);
             p->exec = nullptr;
@@ -2911,8 +3000,7 @@ extern "C" int gmr_pack_multiply(gmr_pack* p, const int* semirings, const void* 
             p->key_lc = lcs;
             p->key_x.assign(dX, dX + n);
             p->key_y.assign(dY, dY + n);
-            p->key_arena.clear();
-            for (auto* e : p->engines) p->key_arena.push_back(e->arena.p);
+            p->key_scratch = scratch_of(p->engines);
             p->launches = total;
         }
         GMR_CUDA(cudaGraphLaunch(p->exec, static_cast<cudaStream_t>(stream)));
