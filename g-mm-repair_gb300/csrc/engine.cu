@@ -41,6 +41,7 @@
 #include "gmr_internal.h"
 #include "async_copy.cuh"
 #include "device_util.cuh"
+#include "sort.cuh"
 
 namespace gmr {
 
@@ -204,6 +205,12 @@ __device__ __forceinline__ void vred(typename S::T* p, const Vec<typename S::T, 
 // launches), 99.5 -> 87.6 us for 20,000 x 5,000 at B = 1.
 __device__ __forceinline__ void dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+}  // namespace gmr
+
+#include "word_fold.cuh"
+
+namespace gmr {
 
 // ------------------------------------------------------------------ kernels
 // Work decomposition: a launch covers right-hand-side tiles
@@ -992,11 +999,12 @@ struct Launch {
     int Bp;       // words per value inside the engine: Bw, or more when padded
     bool padded;  // X and Y rows of Bw words go through padded copies (resolve_launch)
     int push_mode;  // GMR_PUSH_*
+    bool word;      // rules level by level, then every emission in one launch (word_fold.cuh)
     unsigned long long spin_limit;
     std::vector<uint8_t> lv;  // per-launch variant (index = launch slot), empty = uniform emit/chunk
     bool operator==(const Launch& o) const {
         return semiring == o.semiring && B == o.B && Bw == o.Bw && VEC == o.VEC && variant == o.variant &&
-               emit == o.emit && chunk == o.chunk && Bt == o.Bt && Bp == o.Bp && padded == o.padded &&
+               emit == o.emit && chunk == o.chunk && Bt == o.Bt && Bp == o.Bp && padded == o.padded && word == o.word &&
                tile_levels == o.tile_levels &&
                push_mode == o.push_mode && lv == o.lv;
     }
@@ -1046,6 +1054,12 @@ struct gmr_engine {
     // level k has a slot of level k as its source, so level k can push.
     gmr::DevBuf pe_off, pe_row;
     std::vector<uint8_t> push_ok;
+    // One-word fold (word_fold.cuh): the emissions in (chunk, row) order.
+    gmr::DevBuf word_entries, word_seg;
+    gmr::DevBuf word_parts;  // scratch: the copies of Y that chunks add into ((+,x) only)
+    int word_segs = 0, word_blks = 0, word_copies = 1;
+    int64_t word_groups = 0;
+    bool word_ready = false;
     // Left product (y = x^T M): flat edge lists uploaded by gmr_engine_enable_left.
     gmr::DevBuf le_src, le_tgt, le_split, tcol_off, tcol_q;
     std::vector<int64_t> le_off;
@@ -1072,7 +1086,7 @@ struct gmr_engine {
         return {&ops, &op_c, &em_src, &em_row, &seg_row, &seg_start, &term_val, &term_col, &V,
                 &d_lvl_off, &d_em_off, &d_seg_off, &sync, &em_src_c, &em_row_c, &seg_row_c, &seg_start_c,
                 &le_src, &le_tgt, &le_split, &tcol_off, &tcol_q, &em_tcode, &rule_terms, &ops_direct,
-                &pe_off, &pe_row};
+                &pe_off, &pe_row, &word_entries, &word_seg, &word_parts};
     }
 };
 
@@ -1154,14 +1168,15 @@ struct LaunchTimer {
 };
 static thread_local LaunchTimer* t_timer = nullptr;
 
-// A launch of 256 threads per block; pdl: dependent on the kernel before it in
+// A launch; pdl: dependent on the kernel before it in
 // the stream by programmatic dependent launch (that kernel must be one that
 // waits for its own predecessor, or the first of the chain).
 template <class... P>
-static void launch_kernel(void (*kernel)(P...), dim3 grid, size_t smem, cudaStream_t st, bool pdl, P... args) {
+static void launch_kernel_n(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, bool pdl,
+                            P... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(256);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at{};
@@ -1171,6 +1186,10 @@ static void launch_kernel(void (*kernel)(P...), dim3 grid, size_t smem, cudaStre
     cfg.numAttrs = pdl ? 1 : 0;
     GMR_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
+template <class... P>
+static void launch_kernel(void (*kernel)(P...), dim3 grid, size_t smem, cudaStream_t st, bool pdl, P... args) {
+    launch_kernel_n(kernel, grid, 256, smem, st, pdl, args...);
+}
 
 template <class S, int VEC, int GLOG, int DIRK>
 static void launch_level(int emit, dim3 grid, cudaStream_t st, bool pdl, const SweepArgs& s, const LevelArgs& M) {
@@ -1178,6 +1197,32 @@ static void launch_level(int emit, dim3 grid, cudaStream_t st, bool pdl, const S
                    : emit == GMR_EMIT_ROWS ? k_level<S, VEC, GLOG, GMR_EMIT_ROWS, DIRK>
                                            : k_level<S, VEC, GLOG, GMR_EMIT_SEGMENTED, DIRK>;
     launch_kernel(kernel, grid, 0, st, pdl, s, M);
+}
+
+// Copies of Y that the chunks of the one-word fold add into, summed at the end:
+// only (+,x) rounds, and only with many chunks.
+template <class S>
+static int word_copies(const gmr_engine* e) { return std::is_same<S, SPlus>::value ? e->word_copies : 1; }
+
+// The one-launch fold of all emissions (word_fold.cuh) into Y ([copies][rows]).
+template <class S>
+static void launch_word_fold(const gmr_engine* e, void* Y, int copies, cudaStream_t st, bool pdl) {
+    WordFoldArgs w{};
+    w.entries = static_cast<const uint4*>(e->word_entries.p);
+    w.seg = static_cast<const uint32_t*>(e->word_seg.p);
+    w.n_seg = e->word_segs;
+    w.n_blk = e->word_blks;
+    w.n_groups = e->word_groups;
+    w.T = e->T.p;
+    w.arena = e->arena.p;
+    w.n_terms = e->n_terms;
+    w.t_span = word_t_span(e->n_terms);
+    w.n_ops = e->n_ops;
+    w.zero_at = word_zero_at(e->n_terms, e->n_ops);
+    w.Y = Y;
+    w.rows = e->rows;
+    w.copies = copies;
+    launch_kernel_n(k_word_fold<S>, dim3(e->sm_count), kWordThreads, (size_t)(w.zero_at + 1) * 4, st, pdl, w);
 }
 
 // Direct terminal emissions on: the sweep's terminal emissions gather X.
@@ -1212,6 +1257,10 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
     a.G = lc.G;
     a.t0 = 0;
     set_direct(e, a);
+    if (lc.word && word_copies<S>(e) > 1) {  // the copies are zeroed like rows of Y
+        a.Y = e->word_parts.p;
+        a.rows = (int64_t)e->rows * word_copies<S>(e);
+    }
     const int TPB = 256;
     // Not for the timing recorder (it times each launch by itself), for chains
     // with copies and fills between the kernels (staged waits' status), nor
@@ -1236,7 +1285,7 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
         a.x_words = lc.Bw;
     }
     {
-        int64_t items = (e->rows + (e->direct_terms ? e->n_rule_terms : e->n_terms)) * (int64_t)lc.G;
+        int64_t items = (a.rows + (e->direct_terms ? e->n_rule_terms : e->n_terms)) * (int64_t)lc.G;
         dim3 grid(blocks_for(items, lc.ntile), lc.ntile);
         launch_kernel(k_prologue<S, VEC, GLOG>, grid, 0, st, false, a);
         after();
@@ -1384,7 +1433,18 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
     const int D = e->depth;
     const bool staged = any_staged(e, lc) && !t_chain_no_status;
     if (staged) GMR_CUDA(cudaMemsetAsync(e->stage_err(), 0, 8, st));  // the staged waits' error words
-    if (lc.variant == GMR_VARIANT_PLAIN) {
+    if (lc.word) {
+        for (int k = 1; k <= D; ++k) level(k, -1, 0, 1, false);
+        if constexpr (VEC == 1 && GLOG == 0) {
+            launch_word_fold<S>(e, a.Y, word_copies<S>(e), st, pdl);
+            after(a.Y == Y);
+            if (a.Y != Y) {
+                launch_kernel(k_word_sum<S>, dim3(blocks_for(e->rows, 1)), 0, st, pdl, static_cast<const T*>(a.Y),
+                              static_cast<T*>(Y), (int64_t)e->rows, word_copies<S>(e));
+                after();
+            }
+        }
+    } else if (lc.variant == GMR_VARIANT_PLAIN) {
         level(0, 0, 0, lc.ntile, true);  // terminal emissions
         for (int k = 1; k <= D; ++k) {
             level(k, -1, 0, lc.ntile, true);
@@ -1645,6 +1705,11 @@ static Launch resolve_launch(gmr_engine* e, int semiring, int B, const void* X, 
     else if (lc.Bt % 2 == 0 && lc.Bw % 2 == 0 && aligned(8)) lc.VEC = 2;
     else lc.VEC = 1;
     lc.G = lc.Bt / lc.VEC;
+    lc.word = e->word_ready && lc.Bw == 1 && max_vec >= 8 && lc.push_mode == GMR_PUSH_AUTO &&
+              (lc.variant == GMR_VARIANT_GRAPH || lc.variant == GMR_VARIANT_FUSED) &&
+              !(cfg && (cfg->emit_mode || cfg->ops_per_cta > 0)) &&
+              (semiring != GMR_PLUS_TIMES || e->n_em >= kWordMinEmissionsPlus);
+    if (lc.word) lc.lv.clear();  // the tables choose among the per-level folds
     return lc;
 }
 
@@ -1869,6 +1934,60 @@ static void build_push_lists(const gmr_plan& p, gmr_engine& e) {
     upload(row, e.pe_row);
 }
 
+// The (chunk, row) order of the one-word fold (word_fold.cuh), sorted on the
+// GPU from the uploaded emissions.  Not built where it does not pay: graphs
+// with direct terminals (their terminals are no table), too few emissions, or
+// runs too short (kWordMinPerRow).  Without the memory for it the engine keeps
+// the per-level folds.
+static void build_word_fold(gmr_engine& e) {
+    const int64_t E = e.n_em, total = word_t_span(e.n_terms) + e.n_ops;
+    const int64_t chunks = (total + kWordChunk - 1) / kWordChunk, blks = ((int64_t)e.rows + 65535) / 65536;
+    if (e.direct_terms || e.n_ops == 0 || E < kWordMinEmissions || E >= (int64_t)UINT32_MAX - 1 ||
+        (double)E < kWordMinPerRow * (double)chunks * (double)e.rows || chunks * blks > (1 << 20))
+        return;
+    int row_bits = 16;  // at least the 16 bits an entry keeps
+    while ((1ll << row_bits) < e.rows) ++row_bits;
+    int chunk_bits = 1;
+    while ((1ll << chunk_bits) < chunks) ++chunk_bits;
+    const int n_seg = (int)(chunks * blks);
+    try {
+        DevArray<uint64_t> ka(E), kb(E);
+        DevArray<uint32_t> tmp(dev::sort_scratch(E) + 1), first(n_seg + 1);
+        k_word_keys<<<dev::grid_for(E), 256>>>(static_cast<const int32_t*>(e.em_src.p),
+                                               static_cast<const int32_t*>(e.em_row.p), E, word_t_span(e.n_terms),
+                                               row_bits, ka.p);
+        uint64_t *k1 = ka.p, *k2 = kb.p;
+        uint32_t *v1 = nullptr, *v2 = nullptr;
+        dev::radix_sort(k1, k2, v1, v2, E, row_bits + chunk_bits, tmp.p, nullptr);
+        k_word_segments<<<dev::grid_for(n_seg + 1), 256>>>(k1, E, row_bits, (int)blks, n_seg, first.p);
+        GMR_CUDA(cudaGetLastError());
+        std::vector<uint32_t> f((size_t)n_seg + 1), seg((size_t)n_seg + 1, 0);
+        GMR_CUDA(cudaMemcpy(f.data(), first.p, f.size() * 4, cudaMemcpyDeviceToHost));
+        for (int i = 0; i < n_seg; ++i) seg[i + 1] = seg[i] + (f[i + 1] - f[i] + kWordGroup - 1) / kWordGroup;
+        e.word_groups = seg[n_seg];
+        upload(seg, e.word_seg);
+        e.word_entries.ensure((size_t)e.word_groups * kWordGroup * 4);
+        e.word_copies = (int)std::min<int64_t>(kWordMaxCopies, (chunks + kWordChunksPerCopy - 1) / kWordChunksPerCopy);
+        if (e.word_copies > 1) e.word_parts.ensure((size_t)e.rows * e.word_copies * 4);
+        k_word_entries<<<e.sm_count * 8, 256>>>(k1, first.p, static_cast<const uint32_t*>(e.word_seg.p), n_seg,
+                                                e.word_groups, (uint32_t)word_zero_at(e.n_terms, e.n_ops),
+                                                static_cast<uint32_t*>(e.word_entries.p));
+        GMR_CUDA(cudaGetLastError());
+        GMR_CUDA(cudaStreamSynchronize(nullptr));
+    } catch (const Error& err) {
+        if (err.code != GMR_ERR_OOM) throw;
+        e.word_entries.release();
+        e.word_seg.release();
+        e.word_parts.release();
+        return;
+    }
+    for (auto* k : {(const void*)k_word_fold<SPlus>, (const void*)k_word_fold<SBool>, (const void*)k_word_fold<STrop>})
+        GMR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (kWordChunk + 1) * 4));
+    e.word_segs = n_seg;
+    e.word_blks = (int)blks;
+    e.word_ready = true;
+}
+
 extern "C" int gmr_engine_create(const gmr_plan* p, int device, gmr_engine** out) {
     return guarded([&] {
         if (!p || !out) throw Error(GMR_ERR_ARG, "null argument");
@@ -1916,6 +2035,7 @@ extern "C" int gmr_engine_create(const gmr_plan* p, int device, gmr_engine** out
             build_push_lists(*p, *e);
             GMR_CUDA(cudaStreamCreateWithFlags(&e->own_stream, cudaStreamNonBlocking));
             GMR_CUDA(cudaDeviceGetAttribute(&e->sm_count, cudaDevAttrMultiProcessorCount, device));
+            build_word_fold(*e);
         } catch (...) {
             for (auto* b : e->schedule_bufs()) b->release();
             if (e->own_stream) cudaStreamDestroy(e->own_stream);

@@ -10,10 +10,15 @@
 // order, 4 bytes each: the source's place in the chunk and the row's in its
 // block of 65,536 rows, 16 bits each (half the 8 bytes of the level order).
 // Each block takes an equal share of that list, loads the few chunks it spans
-// with coalesced reads, reduces every row's run in registers and issues one
-// reduction per (chunk, row) into Y.  Rows ascend along a warp, so those
-// reductions touch few sectors.  It pays when runs are long enough, that is
-// when a chunk holds about one emission per row or more (kWordMinPerRow).
+// with coalesced reads and reduces every row's run in registers; each run is
+// one reduction into Y.
+//
+// With the gathers out of the way the instruction rate bounds it: a first form
+// with one emission per lane and a shuffle scan over the 32 rows of every warp
+// step issued 96 instructions per 32 emissions.  Here a lane folds four
+// consecutive emissions by itself and only the run at its edges goes through
+// shuffles, and the list is padded with zeroes so that a warp's 128 emissions
+// never cross a (chunk, block of rows): no bounds are checked inside.
 #pragma once
 
 #include <cstdint>
@@ -22,20 +27,45 @@
 
 namespace gmr {
 
-constexpr int kWordChunk = 57344;       // words of values per chunk: 224 KB of a block's 227 KB
-constexpr int kWordThreads = 1024;      // one block per SM
-constexpr int kWordBatch = 8;           // emissions in flight per lane
-constexpr int64_t kWordTermAlign = 64;  // the arena starts at a multiple of this in the value space
+constexpr int kWordChunk = 57344;   // words of values per chunk: 224 KB of a block's 227 KB, and 16-bit places
+constexpr int kWordThreads = 1024;  // one block per SM
+constexpr int kWordGroup = 128;     // emissions per warp step: four per lane
+// Where the fold pays (one multiply as a graph, per-level folds -> this one).
+// Emissions per chunk and row: long enough runs; a chunk of a mosaic holds 1
+// to 60 emissions per row, graphs below 0.25 were not measured faster.
+// Emissions in all: (+,x) loses below about 2 M (5,000 x 2,000, 1.4 M: 40.8 ->
+// 43.4 us) and gains above (100,000 x 600, 3 M: 55.6 -> 50.7; 20,000 x 5,000,
+// 6.6 M: 76 -> 64; 200,000 x 10,000, 109 M: 625 -> 322); the idempotent
+// semirings, whose per-level fold reduces run by run, gain from the start
+// (20,000 nodes of degree 24, (OR,AND): 47 -> 25; 20,000 x 5,000, (min,+):
+// 119 -> 64).
+constexpr double kWordMinPerRow = 0.25;
+constexpr int64_t kWordMinEmissions = 1 << 16, kWordMinEmissionsPlus = 2 << 20;
+// Chunks per copy of Y: a row gets one addition per chunk that emits into it,
+// and the error of that chain grows with its length.
+constexpr int kWordChunksPerCopy = 16, kWordMaxCopies = 16;
+
+// Where the arena starts in the value space: a whole number of 256-byte lines.
+inline int64_t word_t_span(int64_t n_terms) { return (n_terms + 63) / 64 * 64; }
+
+// Place of the zero value: after the largest chunk.
+inline int word_zero_at(int64_t n_terms, int64_t n_ops) {
+    const int64_t total = word_t_span(n_terms) + n_ops;
+    return (int)(total < kWordChunk ? total : kWordChunk);
+}
 
 struct WordFoldArgs {
-    const uint32_t* entries;   // (source in chunk) << 16 | row in block of rows
-    const uint32_t* seg;       // first entry of (chunk, block of rows), then the entry count
+    const uint4* entries;      // groups of 128; an entry: place in the chunk << 16 | row in its block of rows
+    const uint32_t* seg;       // first group of (chunk, block of rows), then the group count
     int n_seg, n_blk;          // chunks x blocks of 65,536 rows; blocks
-    int64_t n_entries;
+    int64_t n_groups;
     const void* T;             // n_terms words
     const void* arena;         // n_ops words
     int64_t n_terms, t_span, n_ops;  // t_span: n_terms rounded up, where the arena starts
-    void* Y;
+    int zero_at;               // place of a zero value, after the largest chunk
+    void* Y;                   // [copies][rows]: chunk c adds into copy c % copies
+    int64_t rows;
+    int copies;
 };
 
 // Chunk `chunk` of the value space into shared memory, 16 bytes per load (both
@@ -58,6 +88,39 @@ __device__ __forceinline__ void load_word_chunk(const WordFoldArgs& a, int chunk
     }
 }
 
+// One warp step: lane l holds emissions 4l .. 4l+3 of 128 in row order.
+template <class S>
+__device__ __forceinline__ void fold_word_group(const uint4 q, const typename S::T* vals, typename S::T* Y, int lane) {
+    using T = typename S::T;
+    constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t r0 = q.x & 0xffffu, r1 = q.y & 0xffffu, r2 = q.z & 0xffffu, r3 = q.w & 0xffffu;
+    const T v0 = vals[q.x >> 16], v1 = vals[q.y >> 16], v2 = vals[q.z >> 16], v3 = vals[q.w >> 16];
+    const bool c1 = r1 == r0, c2 = r2 == r1, c3 = r3 == r2;
+    const T a1 = c1 ? S::oplus(v0, v1) : v1, a2 = c2 ? S::oplus(a1, v2) : v2;
+    T last = c3 ? S::oplus(a2, v3) : v3;  // the run this lane ends with
+    // what the lanes before bring into this lane's first run
+    const uint32_t row_before = __shfl_up_sync(kAll, r3, 1), row_after = __shfl_down_sync(kAll, r0, 1);
+    const bool joined = lane > 0 && row_before == r0;
+    const bool open = lane == 31 || row_after != r3;  // the last run ends here
+    bool through = joined && c1 && c2 && c3;  // one run, continued from the lane before
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        if (!__any_sync(kAll, through)) break;
+        const T o = __shfl_up_sync(kAll, last, d);
+        const bool t = __shfl_up_sync(kAll, (int)through, d);
+        if (through) {
+            last = S::oplus(o, last);
+            through = lane >= d && t;
+        }
+    }
+    const T before = __shfl_up_sync(kAll, last, 1);
+    const T in = joined ? before : S::zero();
+    if (!c1) S::red(Y + r0, S::oplus(v0, in));
+    if (!c2) S::red(Y + r1, c1 ? S::oplus(a1, in) : a1);
+    if (!c3) S::red(Y + r2, c1 && c2 ? S::oplus(a2, in) : a2);
+    if (open) S::red(Y + r3, last);
+}
+
 template <class S>
 __global__ void __launch_bounds__(kWordThreads, 1) k_word_fold(WordFoldArgs a) {
     using T = typename S::T;
@@ -65,61 +128,55 @@ __global__ void __launch_bounds__(kWordThreads, 1) k_word_fold(WordFoldArgs a) {
     T* vals = reinterpret_cast<T*>(word_smem);
     dependents_may_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t per = ((a.n_entries + gridDim.x - 1) / gridDim.x + 31) & ~(int64_t)31;
+    const int64_t per = (a.n_groups + gridDim.x - 1) / gridDim.x;
     int64_t at = (int64_t)blockIdx.x * per;
-    const int64_t end = min(at + per, a.n_entries);
-    int s = 0;  // the segment that holds entry `at`: the last one that starts at or before it
+    const int64_t end = min(at + per, a.n_groups);
+    int s = 0;  // the last (chunk, block of rows) that starts at or before group `at`
     for (int lo = 0, hi = a.n_seg; lo < hi;) {
         const int mid = (lo + hi) >> 1;
-        if (__ldg(a.seg + mid) <= (uint64_t)at) {
+        if ((int64_t)__ldg(a.seg + mid) <= at) {
             s = mid;
             lo = mid + 1;
         } else {
             hi = mid;
         }
     }
+    if (threadIdx.x == 0) vals[a.zero_at] = S::zero();
     wait_for_previous_kernel();
     int loaded = -1;
-    for (; at < end; ++s) {
+    for (; at < end && s < a.n_seg; ++s) {
         const int64_t to = min((int64_t)__ldg(a.seg + s + 1), end);
         if (to <= at) continue;
         const int chunk = s / a.n_blk;
-        T* Y = static_cast<T*>(a.Y) + ((int64_t)(s - chunk * a.n_blk) << 16);
+        T* Y = static_cast<T*>(a.Y) + (chunk % a.copies) * a.rows + ((int64_t)(s - chunk * a.n_blk) << 16);
         if (chunk != loaded) {
             __syncthreads();  // the chunk before is no longer read
             load_word_chunk<T>(a, chunk, vals);
             __syncthreads();
             loaded = chunk;
         }
-        for (int64_t b = at + warp * (32 * kWordBatch); b < to; b += kWordThreads * kWordBatch) {
-            uint32_t e[kWordBatch];
-#pragma unroll
-            for (int u = 0; u < kWordBatch; ++u) {
-                const int64_t i = b + u * 32 + lane;
-                e[u] = i < to ? __ldg(a.entries + i) : 0xffffffffu;  // no source is 0xffff
-            }
-#pragma unroll
-            for (int u = 0; u < kWordBatch; ++u) {
-                const bool valid = e[u] != 0xffffffffu;
-                T v = valid ? vals[e[u] >> 16] : S::zero();
-                const uint32_t row = e[u] & 0xffffu;
-                const uint32_t key = valid ? row : 0x10000u;
-                const uint32_t before = __shfl_up_sync(0xffffffffu, key, 1);
-                const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || before != key);
-                const unsigned above = heads & (0xfffffffeu << lane);
-                const int last = above ? __ffs(above) - 2 : 31;  // last lane of this lane's run
-                // step d is needed while some run is longer than d (d lanes in a row that are no head)
-                unsigned m = ~heads;
-#pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    if (m == 0) break;
-                    const T o = __shfl_down_sync(0xffffffffu, v, d);
-                    if (lane + d <= last) v = S::oplus(v, o);
-                    m &= m >> d;
-                }
-                if (valid && (heads >> lane & 1u)) S::red(Y + row, v);
-            }
+        constexpr int kWarps = kWordThreads / 32;
+        for (int64_t g = at + warp; g < to; g += 2 * kWarps) {  // two groups of loads in flight
+            const bool two = g + kWarps < to;
+            const uint4 q0 = __ldg(a.entries + g * 32 + lane);
+            const uint4 q1 = two ? __ldg(a.entries + (g + kWarps) * 32 + lane) : q0;
+            fold_word_group<S>(q0, vals, Y, lane);
+            if (two) fold_word_group<S>(q1, vals, Y, lane);
         }
+        at = to;
+    }
+}
+
+// Y from its copies.
+template <class S>
+__global__ void __launch_bounds__(256) k_word_sum(const typename S::T* __restrict__ parts, typename S::T* __restrict__ Y,
+                                                  int64_t rows, int copies) {
+    dependents_may_launch();
+    wait_for_previous_kernel();
+    for (int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x; r < rows; r += (int64_t)gridDim.x * 256) {
+        typename S::T v = __ldcg(parts + r);
+        for (int c = 1; c < copies; ++c) v = S::oplus(v, __ldcg(parts + c * rows + r));
+        Y[r] = v;
     }
 }
 
@@ -136,15 +193,9 @@ static __global__ void __launch_bounds__(256) k_word_keys(const int32_t* __restr
     }
 }
 
-static __global__ void __launch_bounds__(256) k_word_entries(const uint64_t* __restrict__ key, int64_t n,
-                                                             uint32_t* __restrict__ entries) {
-    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256)
-        entries[i] = (uint32_t)(key[i] >> 48) << 16 | (uint32_t)(key[i] & 0xffffu);
-}
-
-// seg[s]: the first entry whose (chunk, block of rows) is s or later.
+// first[s]: the first sorted emission whose (chunk, block of rows) is s or later.
 static __global__ void __launch_bounds__(256) k_word_segments(const uint64_t* __restrict__ key, int64_t n, int row_bits,
-                                                              int n_blk, int n_seg, uint32_t* __restrict__ seg) {
+                                                              int n_blk, int n_seg, uint32_t* __restrict__ first) {
     const uint64_t low = (1ull << 48) - 1;
     for (int s = blockIdx.x * 256 + threadIdx.x; s <= n_seg; s += gridDim.x * 256) {
         const uint64_t want = (uint64_t)(s / n_blk) << row_bits | (uint64_t)(s % n_blk) << 16;
@@ -154,7 +205,31 @@ static __global__ void __launch_bounds__(256) k_word_segments(const uint64_t* __
             if ((key[mid] & low) < want) lo = mid + 1;
             else hi = mid;
         }
-        seg[s] = (uint32_t)lo;
+        first[s] = (uint32_t)lo;
+    }
+}
+
+// The entries in whole groups per (chunk, block of rows): one warp per group;
+// past the last emission of its segment an entry is the zero value in the
+// segment's last row.
+static __global__ void __launch_bounds__(256) k_word_entries(const uint64_t* __restrict__ key,
+                                                             const uint32_t* __restrict__ first,
+                                                             const uint32_t* __restrict__ seg, int n_seg, int64_t n_groups,
+                                                             uint32_t zero_at, uint32_t* __restrict__ entries) {
+    const int64_t warps = (int64_t)gridDim.x * 8;
+    for (int64_t g = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); g < n_groups; g += warps) {
+        int lo = 0, hi = n_seg;  // the last segment that starts at or before g (empty ones start with the next)
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if ((int64_t)seg[mid] <= g) lo = mid;
+            else hi = mid;
+        }
+        const uint32_t f0 = first[lo], f1 = first[lo + 1];
+        for (int j = threadIdx.x & 31; j < kWordGroup; j += 32) {
+            const int64_t i = (int64_t)f0 + (g - seg[lo]) * kWordGroup + j;
+            const uint64_t k = key[i < f1 ? i : (int64_t)f1 - 1];
+            entries[g * kWordGroup + j] = (i < f1 ? (uint32_t)(k >> 48) : zero_at) << 16 | (uint32_t)(k & 0xffffu);
+        }
     }
 }
 

@@ -1,0 +1,55 @@
+"""The one-launch fold of 4-byte values (word_fold.cuh): matrices whose emission
+list crosses its edges, against sums over the uncompressed entries.  Tolerance
+for (+,x): 1e-5 relative max-norm of FP64, as everywhere; exact otherwise."""
+import numpy as np
+import pytest
+
+import gmr
+from helpers import INF
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    # more than 65,536 rows (two blocks of rows), many chunks, copies of Y
+    "two_row_blocks": lambda: gmr.gen_mosaic(70001, 610, 64, 0.01, 1e-3, 3),
+    # few long rows: runs far longer than a warp step
+    "long_rows": lambda: gmr.gen_mosaic(41, 30000, 16, 0.02, 0.01, 4),
+    # one chunk, short runs, empty rows at the end of the matrix
+    "graph": lambda: gmr.gen_copy_graph(21000, 12, 0.7, False, 5),
+}
+
+
+@pytest.mark.parametrize("sr", range(3))
+@pytest.mark.parametrize("name", list(CASES))
+def test_word_fold(name, sr):
+    m = CASES[name]()
+    rows, cols, codes, V = m.rows, m.cols, m.codes(), m.values()
+    r = np.repeat(np.arange(rows), np.diff(np.r_[-1, np.flatnonzero(codes == 0)]) - 1)
+    nz = codes[codes != 0].astype(np.int64) - 1
+    c, v = nz % cols, V[nz // cols]
+    eng = gmr.Engine(gmr.Plan.build(gmr.repair(m, device=0), rows, cols, device=0))
+    rng = np.random.default_rng(7)
+    if sr == 0:
+        x = rng.uniform(-1, 1, cols).astype(np.float32)
+        y = eng.multiply(x, 0)[:, 0]
+        ref = np.bincount(r, v * x[c].astype(np.float64), rows)
+        assert np.abs(y - ref).max() <= 1e-5 * np.abs(ref).max()
+    elif sr == 1:
+        B = 17
+        X = rng.random((cols, B)) < 3.0 / cols
+        y = gmr.unpack_bits(eng.multiply(gmr.pack_bits(X), 1, B=B), B)
+        for b in range(B):
+            np.testing.assert_array_equal(y[:, b], np.bincount(r, X[c, b], rows) > 0)
+    else:
+        x = np.where(rng.random(cols) < 0.01, rng.integers(0, 1000, cols), 2**31 - 1).astype(np.int32)
+        y = eng.multiply(x, 2)[:, 0]
+        ref = np.full(rows, INF, dtype=np.int64)
+        np.minimum.at(ref, r, np.where(x[c] >= INF, INF, v.astype(np.int64) + x[c]))
+        np.testing.assert_array_equal(y, ref)
+    # the same multiply again, and with the per-level folds: the plan's other order of the same emissions
+    X1 = np.ones((cols, 1), dtype=np.int32 if sr else np.float32)
+    a, b = eng.multiply(X1, sr, B=1), eng.multiply(X1, sr, B=1, push=gmr.PUSH_NEVER)
+    if sr:
+        np.testing.assert_array_equal(a, b)
+    else:
+        assert np.abs(a - b).max() <= 1e-5 * np.abs(b).max()
