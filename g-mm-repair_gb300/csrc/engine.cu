@@ -1016,7 +1016,7 @@ struct GraphEntry {
     int64_t launches = 0;  // kernel launches inside the graph (one iteration for a fixpoint loop)
     const void* X = nullptr;
     void* Y = nullptr;
-    bool fixpoint = false;  // a whole fixpoint loop (conditional while node) rather than one multiply
+    enum Kind { kRight, kFixpoint, kLeft } kind = kRight;  // kFixpoint: a whole loop (conditional while node)
 };
 
 }  // namespace gmr
@@ -1062,7 +1062,7 @@ struct gmr_engine {
     bool word_ready = false;
     // Left product (y = x^T M): flat edge lists uploaded by gmr_engine_enable_left.
     gmr::DevBuf le_src, le_tgt, le_split, tcol_off, tcol_q;
-    std::vector<int64_t> le_off;
+    std::vector<int64_t> le_off, le_first;  // the plan's offsets; where each range starts on the device
     int64_t n_left_split = 0;
     bool left_ready = false;
     int* status_host = nullptr;                           // pinned copy of the last error words
@@ -1360,11 +1360,22 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
             L.seg_first = e->seg_off[k_em];
             nseg = e->seg_off[k_em + 1] - e->seg_off[k_em];
         }
-        auto em_items_seg = [&](int64_t ne) -> int64_t {  // the segmented fold, chunk 16
+        // A lane group folds its chunk four emissions at a time, each round a
+        // load of indices and then of values: on a level that leaves the GPU
+        // half empty the rounds are the launch's time (4 of them, 3 to 4 us of
+        // a 16-emission chunk), so its chunk is halved while the groups still
+        // fit the GPU at once.
+        auto chunk_of = [&](int64_t ne, int c) {
+            while (c > 4 && (ne + c / 2 - 1) / (c / 2) * lc.G <= (int64_t)e->sm_count * 1024) c /= 2;
+            return (c + 3) & ~3;
+        };
+        auto em_items_seg = [&](int64_t ne) -> int64_t {  // the segmented fold
             if (GLOG == 0) return (ne + 1) / 2;
-            return (ne + 15) / 16 * lc.G;
+            const int c = chunk_of(ne, 16);
+            return (ne + c - 1) / c * lc.G;
         };
         auto em_items = [&](int64_t ne, int64_t ns) -> int64_t {
+            const int chunk = chunk_of(ne, L.em_chunk);
             if (emit == GMR_EMIT_ATOMIC) return ne * lc.G;
             if (emit == GMR_EMIT_ROWS) return ns * lc.G;
             if (GLOG == 0) return (ne + 1) / 2;  // two warp-blocks per warp iteration
@@ -1388,7 +1399,7 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
                     const int eb = ne > 0 ? blocks_for(em_items_seg(ne), nt) : 0;
                     const int ob = (int)std::min<int64_t>((no + R - 1) / R, std::max(1, e->sm_count * ops_cap / nt));
                     M.em_blocks = eb;
-                    M.em_chunk = 16;
+                    M.em_chunk = chunk_of(ne, 16);
                     M.stage_bytes = kStageBytes;
                     M.err = e->stage_err();
                     M.level = k_ops;
@@ -1397,6 +1408,7 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
                     return;
                 }
             }
+            M.em_chunk = chunk_of(ne, M.em_chunk);
             int eb = ne > 0 ? blocks_for(em_items(ne, ns), nt) : 0;
             int ob = no > 0 ? std::min<int>(blocks_for((no * lc.G + 1) / 2, nt),
                                             std::max(1, e->sm_count * ops_cap / nt)) : 0;
@@ -1646,6 +1658,15 @@ static int auto_tile(gmr_engine*, int Bw) {
 // where 36 -> 40 words measured slower.  One multiply, before -> now:
 // 30,001 x 3,001, B = 33: 820 -> 355 us; 50,000 x 5,000: B = 5 287 -> 208 us,
 // B = 7 336 -> 207 us, B = 33 1019 -> 471 us, B = 129 3620 -> 1397 us.
+static bool needs_padding(const gmr_engine* e, int semiring, int Bw, bool aligned16) {
+    if (Bw >= 4 && (Bw % 4 != 0 || !aligned16)) return true;
+    // by choice: the gathers have to outweigh the copy of Y (49,502 x 501, 35
+    // emissions a row, B = 116: 207 us as it is, 232 padded; 1,021 x 645, B = 92: 35 and 44)
+    return Bw % 8 != 0 && (Bw == 12 || (semiring == GMR_PLUS_TIMES && Bw >= 28)) && e->n_em >= (1 << 20) &&
+           e->n_em >= 64 * (int64_t)e->rows;
+}
+static int padded_words(int Bw) { return Bw <= 4 ? 4 : (Bw + 7) / 8 * 8; }
+
 static Launch resolve_launch(gmr_engine* e, int semiring, int B, const void* X, void* Y, const gmr_config* cfg,
                              int max_vec = 8) {
     Launch lc{};
@@ -1673,11 +1694,10 @@ static Launch resolve_launch(gmr_engine* e, int semiring, int B, const void* X, 
     if (lc.variant == GMR_VARIANT_PERSISTENT) bt = lc.Bw;  // one tile: the whole batch in one launch
     lc.Bp = lc.Bw;
     lc.padded = max_vec >= 8 && lc.variant != GMR_VARIANT_PERSISTENT && !tile_asked &&
-                ((lc.Bw >= 4 && (lc.Bw % 4 != 0 || !aligned(16))) ||
-                 (lc.Bw % 8 != 0 && (lc.Bw == 12 || (semiring == GMR_PLUS_TIMES && lc.Bw >= 28))));
+                needs_padding(e, semiring, lc.Bw, aligned(16));
     if (lc.padded) {
         const int nt = (lc.Bw + 127) / 128, per = (lc.Bw + nt - 1) / nt;
-        bt = per <= 4 ? 4 : (per + 7) / 8 * 8;
+        bt = padded_words(per);
         lc.Bp = bt * nt;
     }
     lc.Bt = bt;
@@ -1713,13 +1733,64 @@ static Launch resolve_launch(gmr_engine* e, int semiring, int B, const void* X, 
     return lc;
 }
 
+static void drop_oldest_graph(gmr_engine* e) {
+    if (e->graphs.size() < 8) return;
+    if (e->graphs.front().exec) cudaGraphExecDestroy(e->graphs.front().exec);
+    e->graphs.erase(e->graphs.begin());
+}
+
+// Runs a chain of launches on st and returns their number: launched one by one
+// the first time its arguments are seen, captured into a graph the second
+// time, replayed from then on (the engine remembers 8 sets of arguments).
+// Capturing and instantiating costs more than a small multiply (0.4 ms for 24
+// launches, against 0.1 ms for launching them), which a caller with new
+// buffers on every call would pay each time.
+template <class F>
+static int64_t run_chain(gmr_engine* e, const Launch& lc, GraphEntry::Kind kind, const void* X, void* Y,
+                         cudaStream_t st, F&& chain) {
+    GraphEntry* hit = nullptr;
+    for (auto& g : e->graphs)
+        if (g.kind == kind && g.lc == lc && g.X == X && g.Y == Y) hit = &g;
+    if (!hit) {
+        int64_t n = 0;
+        chain(st, n);
+        drop_oldest_graph(e);
+        GraphEntry ge;
+        ge.kind = kind;
+        ge.lc = lc;
+        ge.X = X;
+        ge.Y = Y;
+        ge.launches = n;
+        e->graphs.push_back(ge);
+        return n;
+    }
+    if (!hit->exec) {
+        cudaGraph_t graph = nullptr;
+        GMR_CUDA(cudaStreamBeginCapture(e->own_stream, cudaStreamCaptureModeThreadLocal));
+        int64_t n = 0;
+        try {
+            chain(e->own_stream, n);
+        } catch (...) {
+            cudaStreamEndCapture(e->own_stream, &graph);
+            if (graph) cudaGraphDestroy(graph);
+            throw;
+        }
+        GMR_CUDA(cudaStreamEndCapture(e->own_stream, &graph));
+        cudaError_t ie = cudaGraphInstantiate(&hit->exec, graph, 0);
+        cudaGraphDestroy(graph);
+        GMR_CUDA(ie);
+        hit->launches = n;
+    }
+    GMR_CUDA(cudaGraphLaunch(hit->exec, st));
+    return hit->launches;
+}
+
 // Grows the value arena and terminal table; cached graphs bake these
 // addresses in, so any reallocation drops them (after the device is idle).
-static void ensure_scratch(gmr_engine* e, int words, bool padded = false) {
+static void ensure_scratch(gmr_engine* e, int words, int64_t padx_rows = 0, int64_t pady_rows = 0) {
     const size_t na = (size_t)std::max<int64_t>(e->n_ops, 1) * words * 4;
     const size_t nt = (size_t)std::max<int64_t>(e->n_terms, 1) * words * 4;
-    const size_t ny = padded ? (size_t)e->rows * words * 4 : 0;
-    const size_t nx = padded && e->direct_terms ? (size_t)e->cols * words * 4 : 0;
+    const size_t ny = (size_t)pady_rows * words * 4, nx = (size_t)padx_rows * words * 4;
     if (na <= e->arena.bytes && nt <= e->T.bytes && ny <= e->padY.bytes && nx <= e->padX.bytes) return;
     GMR_CUDA(cudaDeviceSynchronize());
     for (auto& g : e->graphs)
@@ -1731,6 +1802,10 @@ static void ensure_scratch(gmr_engine* e, int words, bool padded = false) {
     e->padX.ensure(nx);
 }
 
+static void ensure_scratch(gmr_engine* e, const Launch& lc) {  // of a right product
+    ensure_scratch(e, lc.Bp, lc.padded && e->direct_terms ? e->cols : 0, lc.padded ? e->rows : 0);
+}
+
 static void multiply_device(gmr_engine* e, int semiring, const void* X, void* Y, int B, const gmr_config* cfg,
                             cudaStream_t st, bool eager = false) {
     if (semiring < 0 || semiring > 2) throw Error(GMR_ERR_ARG, "unknown semiring");
@@ -1739,41 +1814,11 @@ static void multiply_device(gmr_engine* e, int semiring, const void* X, void* Y,
     if (((uintptr_t)X | (uintptr_t)Y) % 4 != 0) throw Error(GMR_ERR_ARG, "X and Y must be 4-byte aligned");
     Launch lc = resolve_launch(e, semiring, B, X, Y, cfg);
     if (eager && lc.variant == GMR_VARIANT_GRAPH) lc.variant = GMR_VARIANT_FUSED;
-    ensure_scratch(e, lc.Bp, lc.padded);
+    ensure_scratch(e, lc);
     int64_t launches = 0;
     if (lc.variant == GMR_VARIANT_GRAPH) {
-        GraphEntry* hit = nullptr;
-        for (auto& g : e->graphs)
-            if (g.exec && !g.fixpoint && g.lc == lc && g.X == X && g.Y == Y) hit = &g;
-        if (!hit) {
-            if (e->graphs.size() >= 8) {
-                cudaGraphExecDestroy(e->graphs.front().exec);
-                e->graphs.erase(e->graphs.begin());
-            }
-            cudaGraph_t graph = nullptr;
-            GMR_CUDA(cudaStreamBeginCapture(e->own_stream, cudaStreamCaptureModeThreadLocal));
-            int64_t n = 0;
-            try {
-                launch_chain(e, lc, X, Y, e->own_stream, n);
-            } catch (...) {
-                cudaStreamEndCapture(e->own_stream, &graph);
-                if (graph) cudaGraphDestroy(graph);
-                throw;
-            }
-            GMR_CUDA(cudaStreamEndCapture(e->own_stream, &graph));
-            GraphEntry ge;
-            cudaError_t ie = cudaGraphInstantiate(&ge.exec, graph, 0);
-            cudaGraphDestroy(graph);
-            GMR_CUDA(ie);
-            ge.lc = lc;
-            ge.X = X;
-            ge.Y = Y;
-            ge.launches = n;
-            e->graphs.push_back(ge);
-            hit = &e->graphs.back();
-        }
-        GMR_CUDA(cudaGraphLaunch(hit->exec, st));
-        launches = hit->launches;
+        launches = run_chain(e, lc, GraphEntry::kRight, X, Y, st,
+                             [&](cudaStream_t s, int64_t& n) { launch_chain(e, lc, X, Y, s, n); });
     } else if (lc.variant == GMR_VARIANT_PERSISTENT) {
         e->last_persistent = true;
         launch_persistent(e, lc, X, Y, st, launches);
@@ -2426,6 +2471,17 @@ extern "C" void gmr_engine_free(gmr_engine* e) {
 // straddle chunks was set to the semiring zero before the first level and
 // each chunk folds its part into it atomically.  Symbols with thousands of
 // parents or rows are thereby spread over many lane groups.
+//
+// Bound by the L1's tag rate like the right product's folds, so edges are read
+// four at a time (16-byte loads; the device copy of each level's list starts on
+// a multiple of four), values with 32-byte lanes where the right product uses
+// them, odd batches go through padded copies of X and Y, and with one or two
+// words per value a warp folds 128 consecutive edges (fold_runs) instead of
+// each lane walking 16 of its own.
+// The launches follow each other by programmatic dependent launch in a cached
+// graph.  Measured on 50,000 x 5,000 (20 M edges), before -> now: B = 1 342 ->
+// 173 us, B = 32 698 -> 492 us; 3,149 x 575, B = 2 137 -> 59 us; 29,229 x 2,388,
+// B = 10 330 -> 204 us.
 namespace gmr {
 
 struct LeftArgs {
@@ -2442,7 +2498,8 @@ struct LeftArgs {
     const float* V;
     const int32_t* term_val;
     int64_t n_ops, first, count;
-    int Bw, G;
+    int Bw, G;      // words per value (padded), lanes per value
+    int chunk;      // edges per lane group
     bool terminals;  // targets of this launch are terminals (tdown) rather than rules (down)
 };
 
@@ -2452,7 +2509,7 @@ __device__ __forceinline__ Vec<typename S::T, VEC> left_edge_value(const LeftArg
     const bool row = (int64_t)s >= a.n_ops;
     const int64_t pp = s >= 0 ? (int64_t)s : (int64_t)~s;
     const T* base = row ? static_cast<const T*>(a.X) + (pp - a.n_ops) * a.Bw : static_cast<const T*>(a.down) + pp * a.Bw;
-    Vec<T, VEC> v = vload<T, VEC>(base + lane * VEC);
+    Vec<T, VEC> v = vload_rw<T, VEC>(base + lane * VEC);  // down values come from the launch before
     if (a.op_c && s >= 0 && !row) {
         const float c = __ldg(a.op_c + pp);
 #pragma unroll
@@ -2474,6 +2531,8 @@ __device__ __forceinline__ void left_flush(const LeftArgs& a, int32_t u, int lan
 template <class S, int VEC, int GLOG>
 __global__ void __launch_bounds__(256) k_left_zero(LeftArgs a) {
     using T = typename S::T;
+    dependents_may_launch();
+    wait_for_previous_kernel();
     const Span sp = span_of<GLOG>(a.G, blockIdx.x, gridDim.x);
     for_lanes<GLOG>(a.G, sp, [&](int lane) {
     for (int64_t i = sp.u; i < a.count; i += sp.stride) {  // count = straddling targets
@@ -2485,62 +2544,109 @@ __global__ void __launch_bounds__(256) k_left_zero(LeftArgs a) {
 }
 
 template <class S, int VEC, int GLOG>
-__global__ void __launch_bounds__(256) k_left_fold(LeftArgs a) {
+__global__ void __launch_bounds__(256, VEC == 8 ? 4 : 5) k_left_fold(LeftArgs a) {
     using T = typename S::T;
-    const int64_t groups = (a.count + kLeftChunk - 1) / kLeftChunk;
+    dependents_may_launch();
+    wait_for_previous_kernel();
+    const int64_t groups = (a.count + a.chunk - 1) / a.chunk;
     const int32_t* src = a.src + a.first;
     const int32_t* tgt = a.tgt + a.first;
     const Span sp = span_of<GLOG>(a.G, blockIdx.x, gridDim.x);
     for_lanes<GLOG>(a.G, sp, [&](int lane) {
-    for (int64_t g = sp.u; g < groups; g += sp.stride) {
-        const int64_t e0 = g * kLeftChunk, e1 = min(e0 + kLeftChunk, a.count);
-        int32_t cur = __ldg(tgt + e0);
-        bool whole = e0 == 0 || __ldg(tgt + e0 - 1) != cur;  // cur's first edge is in this chunk
-        Vec<T, VEC> acc = vzero<S, VEC>();
-        int64_t e = e0;
-        for (; e + 4 <= e1; e += 4) {
-            int32_t u[4], s4[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                u[j] = __ldg(tgt + e + j);
-                s4[j] = __ldg(src + e + j);
+        for (int64_t g = sp.u; g < groups; g += sp.stride) {
+            const int64_t e0 = g * a.chunk;
+            const int len = (int)min((int64_t)a.chunk, a.count - e0);
+            int32_t cur = __ldg(tgt + e0);
+            bool whole = e0 == 0 || __ldg(tgt + e0 - 1) != cur;  // cur's first edge is in this chunk
+            Vec<T, VEC> acc = vzero<S, VEC>();
+            for (int q = 0; q < len; q += 4) {
+                int4 u = __ldg(reinterpret_cast<const int4*>(tgt + e0 + q));
+                int4 f = __ldg(reinterpret_cast<const int4*>(src + e0 + q));
+                const int n = len - q;  // edges left: past them a repeated source, dropped below
+                if (n < 2) u.y = u.x, f.y = f.x;
+                if (n < 3) u.z = u.y, f.z = f.x;
+                if (n < 4) u.w = u.z, f.w = f.x;
+                const Vec<T, VEC> v0 = left_edge_value<S, VEC>(a, f.x, lane);
+                Vec<T, VEC> v1 = left_edge_value<S, VEC>(a, f.y, lane), v2 = left_edge_value<S, VEC>(a, f.z, lane);
+                Vec<T, VEC> v3 = left_edge_value<S, VEC>(a, f.w, lane);
+                if (n < 2) v1 = vzero<S, VEC>();
+                if (n < 3) v2 = vzero<S, VEC>();
+                if (n < 4) v3 = vzero<S, VEC>();
+                auto fold = [&](int32_t t, const Vec<T, VEC>& v) {
+                    if (t != cur) {
+                        left_flush<S, VEC>(a, cur, lane, whole, acc);
+                        whole = true;
+                        acc = v;
+                        cur = t;
+                    } else {
+                        acc = voplus<S, VEC>(acc, v);
+                    }
+                };
+                fold(u.x, v0);
+                fold(u.y, v1);
+                fold(u.z, v2);
+                fold(u.w, v3);
             }
-            Vec<T, VEC> v[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = left_edge_value<S, VEC>(a, s4[j], lane);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (u[j] != cur) {
-                    left_flush<S, VEC>(a, cur, lane, whole, acc);
-                    whole = true;
-                    acc = v[j];
-                    cur = u[j];
-                } else {
-                    acc = voplus<S, VEC>(acc, v[j]);
-                }
-            }
+            const bool ends = e0 + len == a.count || __ldg(tgt + e0 + len) != cur;  // cur's last edge is in this chunk
+            left_flush<S, VEC>(a, cur, lane, whole && ends, acc);
         }
-        for (; e < e1; ++e) {
-            const int32_t u = __ldg(tgt + e);
-            const Vec<T, VEC> v = left_edge_value<S, VEC>(a, __ldg(src + e), lane);
-            if (u != cur) {
-                left_flush<S, VEC>(a, cur, lane, whole, acc);
-                whole = true;
-                acc = v;
-                cur = u;
-            } else {
-                acc = voplus<S, VEC>(acc, v);
-            }
-        }
-        const bool ends = e1 == a.count || __ldg(tgt + e1) != cur;  // cur's last edge is in this chunk
-        left_flush<S, VEC>(a, cur, lane, whole && ends, acc);
-    }
     });
+}
+
+// One lane per value (one or two words): a warp folds 128 consecutive edges,
+// lane l edges 4l .. 4l+3.  A target is stored when its edges all lie in the
+// 128, else added atomically: 128 is a multiple of every chunk, so every target
+// that straddles two groups also straddles two chunks and starts at zero.
+static constexpr int kLeftGroup = 128;
+
+// Edges per lane group on a level of n edges: kLeftChunk, fewer on levels that
+// do not fill the GPU (the rounds of four edges are their time).
+static int left_chunk(int64_t n) {
+    static_assert(kLeftGroup % kLeftChunk == 0 && kLeftChunk == 16, "chunks divide a group");
+    return n <= (1 << 16) ? 4 : n <= (1 << 18) ? 8 : (int)kLeftChunk;
+}
+
+template <class S, int VEC>
+__global__ void __launch_bounds__(256) k_left_fold_warp(LeftArgs a) {
+    using T = typename S::T;
+    dependents_may_launch();
+    wait_for_previous_kernel();
+    const int lane = threadIdx.x & 31;
+    const int64_t groups = (a.count + kLeftGroup - 1) / kLeftGroup, warps = (int64_t)gridDim.x * 8;
+    const int32_t* src = a.src + a.first;
+    const int32_t* tgt = a.tgt + a.first;
+    for (int64_t g = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); g < groups; g += warps) {
+        const int64_t e0 = g * kLeftGroup, e = e0 + lane * 4, e1 = min(e0 + kLeftGroup, a.count);
+        const int n = (int)min(max(e1 - e, (int64_t)0), (int64_t)4);  // this lane's edges
+        constexpr int32_t kNone = INT32_MAX;
+        int4 u = make_int4(kNone, kNone, kNone, kNone), f = make_int4(0, 0, 0, 0);
+        if (n > 0) {
+            u = __ldg(reinterpret_cast<const int4*>(tgt + e));
+            f = __ldg(reinterpret_cast<const int4*>(src + e));
+        }
+        if (n < 2) u.y = u.x;
+        if (n < 3) u.z = u.y;
+        if (n < 4) u.w = u.z;
+        Vec<T, VEC> v[4];
+        v[0] = n > 0 ? left_edge_value<S, VEC>(a, f.x, 0) : vzero<S, VEC>();
+        v[1] = n > 1 ? left_edge_value<S, VEC>(a, f.y, 0) : vzero<S, VEC>();
+        v[2] = n > 2 ? left_edge_value<S, VEC>(a, f.z, 0) : vzero<S, VEC>();
+        v[3] = n > 3 ? left_edge_value<S, VEC>(a, f.w, 0) : vzero<S, VEC>();
+        // the targets at the group's two ends, and whether they go on beyond it
+        const int32_t tfirst = __ldg(tgt + e0), tlast = __ldg(tgt + e1 - 1);
+        const bool cut_first = e0 > 0 && __ldg(tgt + e0 - 1) == tfirst;
+        const bool cut_last = e1 < a.count && __ldg(tgt + e1) == tlast;
+        fold_runs<S, VEC>(u, v, lane, [&](int32_t t, const Vec<T, VEC>& sum) {
+            if (t != kNone) left_flush<S, VEC>(a, t, 0, !((cut_first && t == tfirst) || (cut_last && t == tlast)), sum);
+        });
+    }
 }
 
 template <class S, int VEC, int GLOG>
 __global__ void __launch_bounds__(256) k_left_columns(LeftArgs a) {
     using T = typename S::T;
+    dependents_may_launch();
+    wait_for_previous_kernel();
     const T* tdown = static_cast<const T*>(a.tdown);
     const Span sp = span_of<GLOG>(a.G, blockIdx.x, gridDim.x);
     for_lanes<GLOG>(a.G, sp, [&](int lane) {
@@ -2548,7 +2654,7 @@ __global__ void __launch_bounds__(256) k_left_columns(LeftArgs a) {
         Vec<T, VEC> acc = vzero<S, VEC>();
         for (int64_t i = __ldg(a.tcol_off + c), i1 = __ldg(a.tcol_off + c + 1); i < i1; ++i) {
             const int32_t q = __ldg(a.tcol_q + i);
-            const Vec<T, VEC> d = vload<T, VEC>(tdown + (int64_t)q * a.Bw + lane * VEC);
+            const Vec<T, VEC> d = vload_rw<T, VEC>(tdown + (int64_t)q * a.Bw + lane * VEC);
             const float v = __ldg(a.V + __ldg(a.term_val + q - 1));
             Vec<T, VEC> l;
 #pragma unroll
@@ -2561,12 +2667,13 @@ __global__ void __launch_bounds__(256) k_left_columns(LeftArgs a) {
 }
 
 template <class S, int VEC, int GLOG>
-static void left_chain_t(gmr_engine* e, int Bw, int G, const void* X, void* Y, cudaStream_t st) {
+static void left_chain_t(gmr_engine* e, const Launch& lc, const void* X, void* Y, cudaStream_t st, int64_t& launches) {
+    using T = typename S::T;
     LeftArgs a{};
     a.down = e->arena.p;
     a.tdown = e->T.p;
-    a.X = X;
-    a.Y = Y;
+    a.X = lc.padded ? e->padX.p : X;
+    a.Y = lc.padded ? e->padY.p : Y;
     a.src = static_cast<const int32_t*>(e->le_src.p);
     a.tgt = static_cast<const int32_t*>(e->le_tgt.p);
     a.split = static_cast<const int32_t*>(e->le_split.p);
@@ -2576,44 +2683,88 @@ static void left_chain_t(gmr_engine* e, int Bw, int G, const void* X, void* Y, c
     a.V = static_cast<const float*>(e->V.p);
     a.term_val = static_cast<const int32_t*>(e->term_val.p);
     a.n_ops = e->n_ops;
-    a.Bw = Bw;
-    a.G = G;
+    a.Bw = lc.Bp;
+    a.G = lc.G;
+    const int64_t G = lc.G;
     auto blocks = [&](int64_t items) {
-        return (int)std::max<int64_t>(1, std::min<int64_t>((items + 255) / 256, (int64_t)e->sm_count * 32));
+        return dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>((items + 255) / 256, (int64_t)e->sm_count * 32)));
+    };
+    bool pdl = false;  // from the second launch on
+    auto launch = [&](auto* kernel, dim3 grid, auto... args) {
+        launch_kernel(kernel, grid, 0, st, pdl, args...);
+        pdl = true;
+        ++launches;
     };
     const int D = e->depth;
+    if (lc.padded)
+        launch(k_restride<T>, blocks((int64_t)e->rows * lc.Bp), static_cast<const T*>(X), static_cast<T*>(e->padX.p),
+               (int64_t)e->rows, lc.Bw, lc.Bw, lc.Bp, T(0));
     a.count = e->n_left_split;
-    if (a.count) k_left_zero<S, VEC, GLOG><<<blocks(a.count * G), 256, 0, st>>>(a);
+    if (a.count) launch(k_left_zero<S, VEC, GLOG>, blocks(a.count * G), a);
     for (int j = D; j >= 0; --j) {  // levels D .. 1 from the top, then the terminals (range D + 1)
         const int k = j ? j : D + 1;
-        a.first = e->le_off[k - 1];
+        a.first = e->le_first[k - 1];
         a.count = e->le_off[k] - e->le_off[k - 1];
         a.terminals = k == D + 1;
+        a.chunk = left_chunk(a.count);
         if (a.count == 0) continue;
-        k_left_fold<S, VEC, GLOG><<<blocks((a.count + kLeftChunk - 1) / kLeftChunk * G), 256, 0, st>>>(a);
+        if constexpr (GLOG == 0 && VEC <= 2)
+            launch(k_left_fold_warp<S, VEC>, blocks((a.count + kLeftGroup - 1) / kLeftGroup * 32), a);
+        else
+            launch(k_left_fold<S, VEC, GLOG>, blocks((a.count + a.chunk - 1) / a.chunk * G), a);
     }
     a.first = 0;
     a.count = e->cols;
-    k_left_columns<S, VEC, GLOG><<<blocks((int64_t)e->cols * G), 256, 0, st>>>(a);
-    GMR_CUDA(cudaGetLastError());
+    launch(k_left_columns<S, VEC, GLOG>, blocks((int64_t)e->cols * G), a);
+    if (lc.padded)
+        launch(k_restride<T>, blocks((int64_t)e->cols * lc.Bw), static_cast<const T*>(e->padY.p), static_cast<T*>(Y),
+               (int64_t)e->cols, lc.Bw, lc.Bp, lc.Bw, T(0));
 }
 
 template <class S>
-static void left_chain_s(gmr_engine* e, int Bw, const void* X, void* Y, cudaStream_t st) {
-    const bool a16 = ((uintptr_t)X % 16 == 0) && ((uintptr_t)Y % 16 == 0);
-    if (Bw % 4 == 0 && a16) {
-        switch (Bw / 4) {
-            case 1: return left_chain_t<S, 4, 0>(e, Bw, 1, X, Y, st);
-            case 2: return left_chain_t<S, 4, 1>(e, Bw, 2, X, Y, st);
-            case 4: return left_chain_t<S, 4, 2>(e, Bw, 4, X, Y, st);
-            case 8: return left_chain_t<S, 4, 3>(e, Bw, 8, X, Y, st);
-            case 16: return left_chain_t<S, 4, 4>(e, Bw, 16, X, Y, st);
-            case 32: return left_chain_t<S, 4, 5>(e, Bw, 32, X, Y, st);
-            default: return left_chain_t<S, 4, -1>(e, Bw, Bw / 4, X, Y, st);
+static void left_chain_s(gmr_engine* e, const Launch& lc, const void* X, void* Y, cudaStream_t st, int64_t& n) {
+    if constexpr (std::is_same<S, SPlus>::value) {
+        if (lc.VEC == 8) {
+            switch (lc.G) {
+                case 4: return left_chain_t<S, 8, 2>(e, lc, X, Y, st, n);
+                case 8: return left_chain_t<S, 8, 3>(e, lc, X, Y, st, n);
+                case 16: return left_chain_t<S, 8, 4>(e, lc, X, Y, st, n);
+                default: return left_chain_t<S, 8, -1>(e, lc, X, Y, st, n);
+            }
         }
     }
-    if (Bw == 1) return left_chain_t<S, 1, 0>(e, Bw, 1, X, Y, st);
-    return left_chain_t<S, 1, -1>(e, Bw, Bw, X, Y, st);
+    if (lc.VEC == 4) {
+        switch (lc.G) {
+            case 1: return left_chain_t<S, 4, 0>(e, lc, X, Y, st, n);
+            case 2: return left_chain_t<S, 4, 1>(e, lc, X, Y, st, n);
+            case 4: return left_chain_t<S, 4, 2>(e, lc, X, Y, st, n);
+            case 8: return left_chain_t<S, 4, 3>(e, lc, X, Y, st, n);
+            case 16: return left_chain_t<S, 4, 4>(e, lc, X, Y, st, n);
+            case 32: return left_chain_t<S, 4, 5>(e, lc, X, Y, st, n);
+            default: return left_chain_t<S, 4, -1>(e, lc, X, Y, st, n);
+        }
+    }
+    if (lc.VEC == 2) return left_chain_t<S, 2, 0>(e, lc, X, Y, st, n);
+    if (lc.G == 1) return left_chain_t<S, 1, 0>(e, lc, X, Y, st, n);
+    return left_chain_t<S, 1, -1>(e, lc, X, Y, st, n);
+}
+
+// Widths and lanes of a left product: the right product's rules, one tile.
+static Launch resolve_left(gmr_engine* e, int semiring, int B, const void* X, void* Y) {
+    Launch lc{};
+    lc.semiring = semiring;
+    lc.B = B;
+    lc.Bw = words_per_slot(semiring, B);
+    auto aligned = [&](size_t al) { return ((uintptr_t)X % al == 0) && ((uintptr_t)Y % al == 0); };
+    lc.padded = needs_padding(e, semiring, lc.Bw, aligned(16));
+    lc.Bt = lc.Bp = lc.padded ? padded_words(lc.Bw) : lc.Bw;
+    lc.ntile = 1;
+    if (semiring == GMR_PLUS_TIMES && lc.Bp % 8 == 0 && lc.Bp >= 32 && (lc.padded || aligned(32))) lc.VEC = 8;
+    else if (lc.Bp % 4 == 0) lc.VEC = 4;  // not padded: 16-byte aligned
+    else if (lc.Bp == 2 && aligned(8)) lc.VEC = 2;
+    else lc.VEC = 1;
+    lc.G = lc.Bp / lc.VEC;
+    return lc;
 }
 
 }  // namespace gmr
@@ -2627,13 +2778,40 @@ extern "C" int gmr_engine_enable_left(gmr_engine* e, gmr_plan* p) {
         if (rc != GMR_OK) throw Error(rc, gmr_last_error());
         std::lock_guard<std::mutex> lk(e->mu);
         DeviceGuard dg(e->device);
-        upload(p->le_src, e->le_src);
-        upload(p->le_tgt, e->le_tgt);
-        upload(p->le_split, e->le_split);
+        {
+            // each level's list from a multiple of four on: edges are read in aligned quads
+            const int D = e->depth;
+            std::vector<int64_t> first((size_t)D + 2, 0);
+            for (int k = 1; k <= D + 1; ++k) first[k] = (first[k - 1] + (p->le_off[k] - p->le_off[k - 1]) + 3) & ~(int64_t)3;
+            e->le_src.ensure((size_t)first[D + 1] * 4 + 16);
+            e->le_tgt.ensure((size_t)first[D + 1] * 4 + 16);
+            for (int k = 1; k <= D + 1; ++k) {
+                const size_t n = (size_t)(p->le_off[k] - p->le_off[k - 1]) * 4;
+                if (!n) continue;
+                GMR_CUDA(cudaMemcpy(static_cast<int32_t*>(e->le_src.p) + first[k - 1], p->le_src.data() + p->le_off[k - 1], n,
+                                    cudaMemcpyHostToDevice));
+                GMR_CUDA(cudaMemcpy(static_cast<int32_t*>(e->le_tgt.p) + first[k - 1], p->le_tgt.data() + p->le_off[k - 1], n,
+                                    cudaMemcpyHostToDevice));
+            }
+            e->le_first = std::move(first);
+        }
+        // targets whose edges straddle the chunks used here (the plan's list is for kLeftChunk throughout)
+        std::vector<int32_t> split;
+        for (int k = 1; k <= e->depth + 1; ++k) {
+            const int64_t lo = p->le_off[k - 1], hi = p->le_off[k], c = left_chunk(hi - lo);
+            int32_t before = -1;
+            for (int64_t b = lo + c; b < hi; b += c) {  // chunk boundaries: the target on both sides
+                const int32_t t = p->le_tgt[b];
+                if (t != p->le_tgt[b - 1] || t == before) continue;
+                split.push_back(k <= e->depth ? t : (int32_t)(e->n_ops + t));
+                before = t;
+            }
+        }
+        upload(split, e->le_split);
         upload(p->tcol_off, e->tcol_off);
         upload(p->tcol_q, e->tcol_q);
         e->le_off = p->le_off;
-        e->n_left_split = (int64_t)p->le_split.size();
+        e->n_left_split = (int64_t)split.size();
         e->left_ready = true;
     });
 }
@@ -2649,13 +2827,14 @@ extern "C" int gmr_engine_multiply_left(gmr_engine* e, int semiring, const void*
         if (((uintptr_t)dX | (uintptr_t)dY) % 4 != 0) throw Error(GMR_ERR_ARG, "X and Y must be 4-byte aligned");
         std::lock_guard<std::mutex> lk(e->mu);
         DeviceGuard dg(e->device);
-        const int Bw = words_per_slot(semiring, B);
-        ensure_scratch(e, Bw);
-        cudaStream_t st = static_cast<cudaStream_t>(stream);
-        if (semiring == GMR_PLUS_TIMES) left_chain_s<SPlus>(e, Bw, dX, dY, st);
-        else if (semiring == GMR_BOOLEAN) left_chain_s<SBool>(e, Bw, dX, dY, st);
-        else left_chain_s<STrop>(e, Bw, dX, dY, st);
-        e->last_launches = e->depth + 2 + (e->n_left_split ? 1 : 0);
+        const Launch lc = resolve_left(e, semiring, B, dX, dY);
+        ensure_scratch(e, lc.Bp, lc.padded ? e->rows : 0, lc.padded ? e->cols : 0);
+        e->last_launches = run_chain(e, lc, GraphEntry::kLeft, dX, dY, static_cast<cudaStream_t>(stream),
+                                     [&](cudaStream_t st, int64_t& n) {
+                                         if (semiring == GMR_PLUS_TIMES) left_chain_s<SPlus>(e, lc, dX, dY, st, n);
+                                         else if (semiring == GMR_BOOLEAN) left_chain_s<SBool>(e, lc, dX, dY, st, n);
+                                         else left_chain_s<STrop>(e, lc, dX, dY, st, n);
+                                     });
     });
 }
 
@@ -2702,18 +2881,15 @@ __global__ void k_set_i32(int* p, int v) { *p = v; }
 static GraphEntry* fixpoint_graph(gmr_engine* e, const Launch& lc, int semiring, void* X, void* Y, int64_t n,
                                   int* flag, int* count, const int* max_iters) {
     for (auto& g : e->graphs)
-        if (g.exec && g.fixpoint && g.lc == lc && g.X == X && g.Y == Y) return &g;
-    if (e->graphs.size() >= 8) {
-        cudaGraphExecDestroy(e->graphs.front().exec);
-        e->graphs.erase(e->graphs.begin());
-    }
+        if (g.exec && g.kind == GraphEntry::kFixpoint && g.lc == lc && g.X == X && g.Y == Y) return &g;
+    drop_oldest_graph(e);
     cudaGraph_t graph = nullptr;
     GMR_CUDA(cudaGraphCreate(&graph, 0));
     GraphEntry ge;
     ge.lc = lc;
     ge.X = X;
     ge.Y = Y;
-    ge.fixpoint = true;
+    ge.kind = GraphEntry::kFixpoint;
     try {
         cudaGraphConditionalHandle h;
         GMR_CUDA(cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault));
@@ -2781,7 +2957,7 @@ extern "C" int gmr_engine_fixpoint(gmr_engine* e, int semiring, void* dX, void* 
         if (max_iters == 0) return;
         Launch lc = resolve_launch(e, semiring, B, dX, dY, nullptr);
         if (lc.variant == GMR_VARIANT_GRAPH || lc.variant == GMR_VARIANT_PERSISTENT) lc.variant = GMR_VARIANT_FUSED;
-        ensure_scratch(e, lc.Bp, lc.padded);
+        ensure_scratch(e, lc);
         const int64_t n = (int64_t)e->rows * lc.Bw;
         e->sync.ensure(64);
         int* flag = reinterpret_cast<int*>(static_cast<unsigned char*>(e->sync.p) + 8);
@@ -3078,7 +3254,7 @@ extern "C" int gmr_pack_multiply(gmr_pack* p, const int* semirings, const void* 
             if (B[i] < 1) throw Error(GMR_ERR_ARG, "B must be >= 1");
             if (((uintptr_t)dX[i] | (uintptr_t)dY[i]) % 4 != 0) throw Error(GMR_ERR_ARG, "misaligned X or Y");
             Launch lc = resolve_launch(e, semirings[i], B[i], dX[i], dY[i], nullptr, one_kernel ? 4 : 8);
-            ensure_scratch(e, lc.Bp, lc.padded);
+            ensure_scratch(e, lc);
             lcs.push_back(lc);
         }
         p->last_persistent = false;

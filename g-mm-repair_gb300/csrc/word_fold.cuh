@@ -88,37 +88,52 @@ __device__ __forceinline__ void load_word_chunk(const WordFoldArgs& a, int chunk
     }
 }
 
-// One warp step: lane l holds emissions 4l .. 4l+3 of 128 in row order.
-template <class S>
-__device__ __forceinline__ void fold_word_group(const uint4 q, const typename S::T* vals, typename S::T* Y, int lane) {
-    using T = typename S::T;
+// One warp step of a segmented fold: lane l holds items 4l .. 4l+3 of 128,
+// items with equal keys are contiguous, and flush(key, sum) is called once per
+// run.  A lane folds its own four; a run that crosses lanes is carried from
+// the lane before (a scan over the lanes that are one run throughout, as many
+// steps as the longest such stretch needs).
+template <class S, int VEC, class Flush>
+__device__ __forceinline__ void fold_runs(const int4 k, const Vec<typename S::T, VEC> (&v)[4], int lane, Flush&& flush) {
+    using V = Vec<typename S::T, VEC>;
     constexpr unsigned kAll = 0xffffffffu;
-    const uint32_t r0 = q.x & 0xffffu, r1 = q.y & 0xffffu, r2 = q.z & 0xffffu, r3 = q.w & 0xffffu;
-    const T v0 = vals[q.x >> 16], v1 = vals[q.y >> 16], v2 = vals[q.z >> 16], v3 = vals[q.w >> 16];
-    const bool c1 = r1 == r0, c2 = r2 == r1, c3 = r3 == r2;
-    const T a1 = c1 ? S::oplus(v0, v1) : v1, a2 = c2 ? S::oplus(a1, v2) : v2;
-    T last = c3 ? S::oplus(a2, v3) : v3;  // the run this lane ends with
-    // what the lanes before bring into this lane's first run
-    const uint32_t row_before = __shfl_up_sync(kAll, r3, 1), row_after = __shfl_down_sync(kAll, r0, 1);
-    const bool joined = lane > 0 && row_before == r0;
-    const bool open = lane == 31 || row_after != r3;  // the last run ends here
-    bool through = joined && c1 && c2 && c3;  // one run, continued from the lane before
+    auto shfl_up = [](const V& x, int d) {
+        V o;
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) o.v[j] = __shfl_up_sync(kAll, x.v[j], d);
+        return o;
+    };
+    const bool c1 = k.y == k.x, c2 = k.z == k.y, c3 = k.w == k.z;
+    const V a1 = c1 ? voplus<S, VEC>(v[0], v[1]) : v[1], a2 = c2 ? voplus<S, VEC>(a1, v[2]) : v[2];
+    V last = c3 ? voplus<S, VEC>(a2, v[3]) : v[3];  // the run this lane ends with
+    const int32_t key_before = __shfl_up_sync(kAll, k.w, 1), key_after = __shfl_down_sync(kAll, k.x, 1);
+    const bool joined = lane > 0 && key_before == k.x;  // the first run goes on from the lane before
+    const bool open = lane == 31 || key_after != k.w;   // the last run ends here
+    bool through = joined && c1 && c2 && c3;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
         if (!__any_sync(kAll, through)) break;
-        const T o = __shfl_up_sync(kAll, last, d);
+        const V o = shfl_up(last, d);
         const bool t = __shfl_up_sync(kAll, (int)through, d);
         if (through) {
-            last = S::oplus(o, last);
+            last = voplus<S, VEC>(o, last);
             through = lane >= d && t;
         }
     }
-    const T before = __shfl_up_sync(kAll, last, 1);
-    const T in = joined ? before : S::zero();
-    if (!c1) S::red(Y + r0, S::oplus(v0, in));
-    if (!c2) S::red(Y + r1, c1 ? S::oplus(a1, in) : a1);
-    if (!c3) S::red(Y + r2, c1 && c2 ? S::oplus(a2, in) : a2);
-    if (open) S::red(Y + r3, last);
+    const V before = shfl_up(last, 1);
+    const V in = joined ? before : vzero<S, VEC>();
+    if (!c1) flush(k.x, voplus<S, VEC>(v[0], in));
+    if (!c2) flush(k.y, c1 ? voplus<S, VEC>(a1, in) : a1);
+    if (!c3) flush(k.z, c1 && c2 ? voplus<S, VEC>(a2, in) : a2);
+    if (open) flush(k.w, last);
+}
+
+template <class S>
+__device__ __forceinline__ void fold_word_group(const uint4 q, const typename S::T* vals, typename S::T* Y, int lane) {
+    using T = typename S::T;
+    const int4 row = make_int4(q.x & 0xffff, q.y & 0xffff, q.z & 0xffff, q.w & 0xffff);
+    const Vec<T, 1> v[4] = {{vals[q.x >> 16]}, {vals[q.y >> 16]}, {vals[q.z >> 16]}, {vals[q.w >> 16]}};
+    fold_runs<S, 1>(row, v, lane, [&](int32_t r, const Vec<T, 1>& sum) { S::red(Y + r, sum.v[0]); });
 }
 
 template <class S>

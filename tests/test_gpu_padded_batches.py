@@ -54,3 +54,30 @@ def test_misaligned_pointers(offset, B):
     assert (y[:offset] == 7).all() and (y[offset + m.rows * B:] == 7).all()
     sched = O.RefSchedule(g.alpha, g.rules(), g.C())
     check(0, y[offset:offset + m.rows * B].reshape(m.rows, B), oracle_columns(sched, 0, g.values(), X, m.rows, m.cols))
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("sr", range(3))
+@pytest.mark.parametrize("words", [1, 2, 3, 4, 5, 8, 12, 31, 32, 33, 96, 130, 1030])
+def test_left_widths(weighted, sr, words):
+    """The left product at every lane layout: one and two words (warp folds of
+    128 edges), odd widths, 32-byte lanes, more lanes than a block's threads."""
+    import torch
+    from helpers import brute_left
+
+    if sr == 1 and words > 5:
+        pytest.skip("bit-packed: the word widths above cover the layout")
+    m, g = _grammar(weighted)
+    B = words * 32 - 5 if sr == 1 else words
+    plan = gmr.Plan.build(g, m.rows, m.cols)
+    eng = gmr.Engine(plan)
+    eng.enable_left(plan)
+    X = random_X(sr, m.rows, B, words)
+    dX = torch.from_numpy(engine_inputs(sr, X).view(np.int32)).cuda()
+    ref = brute_left(m.codes(), g.values(), X, m.rows, m.cols, sr)
+    for _ in range(3):  # launched one by one, captured, replayed
+        dY = torch.full((m.cols, dX.shape[1]), 7, dtype=torch.int32, device="cuda")
+        eng.multiply_left_device(sr, dX.data_ptr(), dY.data_ptr(), B)
+        torch.cuda.synchronize()
+    Y = dY.cpu().numpy().view(np.uint32 if sr == 1 else np.float32 if sr == 0 else np.int32)
+    check(sr, engine_outputs(sr, Y, B), ref)
