@@ -497,55 +497,50 @@ __device__ __forceinline__ void do_emits_atomic(const SweepArgs& a, const LevelA
     });
 }
 
-// Warp-segmented emits when G == 1: lane = emission; rows are sorted, so
-// equal rows are contiguous lanes; each segment is reduced in registers
-// (shuffles for (+,x), __reduce_*_sync for OR / min) and its first lane issues
-// one atomic per word.  Two warp-blocks are in flight per iteration.
-template <class S, int VEC>
-__device__ __forceinline__ Vec<typename S::T, VEC> warp_segment_reduce(Vec<typename S::T, VEC> v, unsigned peers,
-                                                                       int lane) {
-    using T = typename S::T;
-    Vec<T, VEC> tot;
-    if constexpr (std::is_same<S, SBool>::value) {
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) tot.v[j] = __reduce_or_sync(peers, v.v[j]);
-    } else if constexpr (std::is_same<S, STrop>::value) {
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) tot.v[j] = __reduce_min_sync(peers, v.v[j]);
-    } else {
-        const int last = 31 - __clz(peers);  // segments are contiguous lanes
-        tot = v;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-#pragma unroll
-            for (int j = 0; j < VEC; ++j) {
-                T o = __shfl_down_sync(0xffffffffu, tot.v[j], d);
-                if (lane + d <= last) tot.v[j] = S::oplus(tot.v[j], o);
-            }
-        }
-    }
-    return tot;
-}
-
+// Warp-segmented emits when G == 1: a warp folds 128 consecutive emissions,
+// lane l emissions 4l .. 4l+3 (aligned on the emission index: two 16-byte index
+// loads and four values in flight per lane), and issues one reduction per row
+// run (fold_runs).  One emission per lane, with the rows grouped by
+// __match_any_sync and reduced by __reduce_*_sync or 5 shuffles, spent its time
+// on those: a step of 32 frontiers on 8 M nodes 1090 -> 691 us, a (min,+) step
+// on 2 M nodes 307 -> 212 us.  Levels whose emissions fit the GPU's lanes at once
+// (em_chunk = 1) keep one per lane, with twice the warps and a shorter chain:
+// 2,000 x 1,000, (+,x) 34.2 us with four per lane throughout, 29.4 with one.
 template <class S, int VEC, bool CG = false, bool DIR = false>
 __device__ __forceinline__ void do_emits_warp(const SweepArgs& a, const LevelArgs& L, int tile, const Span& sp) {
     using T = typename S::T;
     const Values<S, VEC, CG> val(a, tile);
     const int lane = threadIdx.x & 31;
-    const int64_t n = L.n_em, stride = sp.stride;  // one lane per unit: sp.u = this thread's emission
-    for (int64_t base = sp.u - lane; base < n; base += 2 * stride) {  // warp-uniform trip count
-        const int64_t ea = base + lane, eb = base + stride + lane;
-        const bool va = ea < n, vb = eb < n;
-        const int32_t ra = va ? __ldg(L.em_row + L.em_first + ea) : -1 - lane;
-        const int32_t rb = vb ? __ldg(L.em_row + L.em_first + eb) : -1 - lane;
-        const int32_t sa = va ? __ldg(L.em_src + L.em_first + ea) : -1;
-        const int32_t sb = vb ? __ldg(L.em_src + L.em_first + eb) : -1;
-        Vec<T, VEC> xa = val.template get_em<DIR>(sa, 0), xb = val.template get_em<DIR>(sb, 0);  // -1: zero
-        const unsigned pa = __match_any_sync(0xffffffffu, ra), pb = __match_any_sync(0xffffffffu, rb);
-        Vec<T, VEC> ta = warp_segment_reduce<S, VEC>(xa, pa, lane);
-        Vec<T, VEC> tb = warp_segment_reduce<S, VEC>(xb, pb, lane);
-        if (va && lane == __ffs(pa) - 1) vred<S, VEC>(yptr<T>(a, ra, tile, 0, VEC), ta);
-        if (vb && lane == __ffs(pb) - 1) vred<S, VEC>(yptr<T>(a, rb, tile, 0, VEC), tb);
+    const int64_t first = L.em_first, end = first + L.n_em, base = first & ~(int64_t)3;
+    if (L.em_chunk == 1) {
+        for (int64_t w = first + sp.u - lane; w < end; w += sp.stride) {
+            const int64_t e = w + lane;
+            const int32_t r = e < end ? __ldg(L.em_row + e) : -1, s = e < end ? __ldg(L.em_src + e) : -1;
+            const Vec<T, VEC> v = fold_lanes<S, VEC>(r, val.template get_em<DIR>(s, 0), lane);
+            const int32_t before = __shfl_up_sync(0xffffffffu, r, 1);
+            if (r >= 0 && (lane == 0 || before != r)) vred<S, VEC>(yptr<T>(a, r, tile, 0, VEC), v);
+        }
+        return;
+    }
+    // one lane per unit: sp.u is this thread's place in the grid, four emissions each
+    for (int64_t w = base + (sp.u - lane) * 4; w < end; w += sp.stride * 4) {  // warp-uniform trip count
+        const int64_t e = w + lane * 4;
+        int4 r = make_int4(-1, -1, -1, -1), s = r;  // -1: the zero value, in no row
+        if (e < end) {
+            r = __ldg(reinterpret_cast<const int4*>(L.em_row + e));
+            s = __ldg(reinterpret_cast<const int4*>(L.em_src + e));
+            if (e < first || e + 4 > end) {
+                if (e < first) r.x = s.x = -1;
+                if (e + 1 < first || e + 1 >= end) r.y = s.y = -1;
+                if (e + 2 < first || e + 2 >= end) r.z = s.z = -1;
+                if (e + 3 >= end) r.w = s.w = -1;
+            }
+        }
+        const Vec<T, VEC> v[4] = {val.template get_em<DIR>(s.x, 0), val.template get_em<DIR>(s.y, 0),
+                                  val.template get_em<DIR>(s.z, 0), val.template get_em<DIR>(s.w, 0)};
+        fold_runs<S, VEC>(r, v, lane, [&](int32_t row, const Vec<T, VEC>& sum) {
+            if (row >= 0) vred<S, VEC>(yptr<T>(a, row, tile, 0, VEC), sum);
+        });
     }
 }
 
@@ -1366,19 +1361,24 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
         // a 16-emission chunk), so its chunk is halved while the groups still
         // fit the GPU at once.
         auto chunk_of = [&](int64_t ne, int c) {
-            while (c > 4 && (ne + c / 2 - 1) / (c / 2) * lc.G <= (int64_t)e->sm_count * 1024) c /= 2;
-            return (c + 3) & ~3;
+            if constexpr (GLOG == 0) {
+                return ne <= (int64_t)e->sm_count * 2048 ? 1 : 4;  // emissions per lane
+            } else {
+                while (c > 4 && (ne + c / 2 - 1) / (c / 2) * lc.G <= (int64_t)e->sm_count * 1024) c /= 2;
+                return (c + 3) & ~3;
+            }
         };
         auto em_items_seg = [&](int64_t ne) -> int64_t {  // the segmented fold
-            if (GLOG == 0) return (ne + 1) / 2;
             const int c = chunk_of(ne, 16);
+            if (GLOG == 0) return c == 1 ? ne : (ne + 6) / 4;  // one per lane, or four from an aligned start
+
             return (ne + c - 1) / c * lc.G;
         };
         auto em_items = [&](int64_t ne, int64_t ns) -> int64_t {
             const int chunk = chunk_of(ne, L.em_chunk);
             if (emit == GMR_EMIT_ATOMIC) return ne * lc.G;
             if (emit == GMR_EMIT_ROWS) return ns * lc.G;
-            if (GLOG == 0) return (ne + 1) / 2;  // two warp-blocks per warp iteration
+            if (GLOG == 0) return chunk == 1 ? ne : (ne + 6) / 4;
             return (ne + chunk - 1) / chunk * lc.G;
         };
         auto go = [&](const LevelArgs& base, int64_t no, int64_t ne, int64_t ns, bool mark) {
@@ -3138,7 +3138,7 @@ static void pack_level_blocks(const gmr_engine* e, const PackGrammar& g, int k, 
     if (k > e->depth + 1) return;
     const int64_t ne = e->em_off[k] - e->em_off[k - 1];
     const int64_t no = k <= e->depth ? e->lvl_off[k] - e->lvl_off[k - 1] : 0;
-    if (ne > 0) *eb = blocks(lane_per_unit ? (ne + 1) / 2 : (ne + 15) / 16 * G);
+    if (ne > 0) *eb = blocks(lane_per_unit ? (ne + 6) / 4 : (ne + 15) / 16 * G);
     if (no > 0) *ob = blocks((no * G + 1) / 2);
 }
 

@@ -128,6 +128,28 @@ __device__ __forceinline__ void fold_runs(const int4 k, const Vec<typename S::T,
     if (open) flush(k.w, last);
 }
 
+// The same with one item per lane: the sum of its run in the run's first lane.
+template <class S, int VEC>
+__device__ __forceinline__ Vec<typename S::T, VEC> fold_lanes(int32_t key, Vec<typename S::T, VEC> v, int lane) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int32_t before = __shfl_up_sync(kAll, key, 1);
+    const unsigned heads = __ballot_sync(kAll, lane == 0 || before != key);
+    const unsigned above = heads & (0xfffffffeu << lane);
+    const int last = above ? __ffs(above) - 2 : 31;  // last lane of this lane's run
+    unsigned m = ~heads;  // step d is needed while some run is longer than d: d lanes in a row that start none
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        if (m == 0) break;
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) {
+            const typename S::T o = __shfl_down_sync(kAll, v.v[j], d);
+            if (lane + d <= last) v.v[j] = S::oplus(v.v[j], o);
+        }
+        m &= m >> d;
+    }
+    return v;
+}
+
 template <class S>
 __device__ __forceinline__ void fold_word_group(const uint4 q, const typename S::T* vals, typename S::T* Y, int lane) {
     using T = typename S::T;
