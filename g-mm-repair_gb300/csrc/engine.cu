@@ -41,6 +41,7 @@
 #include "gmr_internal.h"
 #include "async_copy.cuh"
 #include "device_util.cuh"
+#include "emission_orders.cuh"
 #include "sort.cuh"
 
 namespace gmr {
@@ -1310,6 +1311,11 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
             chunk = kEmitVariants[v % kNumEmitVariants].chunk;
             ops_cap = kOpsCtasPerSm[(v / kNumEmitVariants) % 2];
             by_chunk = v >= 2 * kNumEmitVariants;
+            // with one lane per value the warp fold beats the row-owned and the
+            // atomic one on every level (98,160 x 7,210, 128 Boolean columns: 416
+            // us a multiply against 553 and 1870; (+,x) B = 4: 402, 555, 706), and
+            // tables made before it was the fastest still ask for those
+            if (GLOG == 0) emit = GMR_EMIT_SEGMENTED;
         }
         if (lc.variant == GMR_VARIANT_PLAIN) emit = GMR_EMIT_ATOMIC;
         // level k_em pushed its emissions in its own launch: nothing to fold
@@ -1362,7 +1368,7 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
         // fit the GPU at once.
         auto chunk_of = [&](int64_t ne, int c) {
             if constexpr (GLOG == 0) {
-                return ne <= (int64_t)e->sm_count * 2048 ? 1 : 4;  // emissions per lane
+                return ne <= (int64_t)e->sm_count * (std::is_same<S, SPlus>::value ? 8192 : 2048) ? 1 : 4;  // per lane
             } else {
                 while (c > 4 && (ne + c / 2 - 1) / (c / 2) * lc.G <= (int64_t)e->sm_count * 1024) c /= 2;
                 return (c + 3) & ~3;
@@ -1854,67 +1860,99 @@ struct Nvml {
 
 using namespace gmr;
 
+static int bits_for(uint64_t x) { return x == 0 ? 0 : 64 - __builtin_clzll(x); }
+
+// Builds one of the engine's other emission orders; without the device memory
+// for it the engine goes without (every multiply has the level order).
+template <class F>
+static bool build_order(F&& f) {
+    try {
+        f();
+        return true;
+    } catch (const Error& err) {
+        if (err.code != GMR_ERR_OOM) throw;
+        return false;
+    }
+}
+
 // The chunked emission order (see gmr_engine::ch_*), built when some level
-// has more than one source chunk: a stable counting sort of each level's
-// (row, source)-ordered emissions by source chunk, then row segments per chunk.
+// has more than one source chunk: each level's (row, source)-ordered emissions
+// stably sorted by source chunk, then row segments per chunk.
 // The chunk size is kChunkSlots unless the environment variable
 // GMR_CHUNK_SLOTS (read when the engine is created) sets another one.
 static void build_chunked_emissions(const gmr_plan& p, gmr_engine& e) {
     const int D = p.depth;
-    int64_t kChunkSlots = gmr::kChunkSlots;
+    int64_t slots = gmr::kChunkSlots;
     if (const char* env = std::getenv("GMR_CHUNK_SLOTS")) {
         long long v = std::atoll(env);
-        if (v >= 1) kChunkSlots = v;
+        if (v >= 1) slots = v;
     }
-    e.chunk_slots = kChunkSlots;
+    e.chunk_slots = slots;
     bool any = false;
     for (int k = 0; k <= D && !any; ++k) {
         const int64_t width = k == 0 ? p.n_terms() : p.lvl_off[k] - p.lvl_off[k - 1];
-        any = width > kChunkSlots && p.em_off[k + 1] > p.em_off[k];
+        any = width > slots && p.em_off[k + 1] > p.em_off[k];
     }
     if (!any) return;
     const int64_t E = (int64_t)p.em_src.size();
-    std::vector<int32_t> src(E), row(E), srow;
-    std::vector<int64_t> sstart;
-    e.ch_off.assign(D + 2, 0);
-    e.ch_em.clear();
-    e.ch_seg.clear();
+    std::vector<int64_t> base((size_t)D + 2, 0);  // a level's sources are its slots, or terminals
     for (int k = 0; k <= D; ++k) {
-        e.ch_off[k] = (int64_t)e.ch_em.size();
-        const int64_t lo = p.em_off[k], hi = p.em_off[k + 1];
-        if (hi == lo) continue;
-        const int64_t base = k == 0 ? 0 : p.lvl_off[k - 1];
-        auto chunk_of = [&](int32_t c) { return (c >= 0 ? (int64_t)c - base : -(int64_t)c - 1) / kChunkSlots; };
-        int64_t nc = 0;
-        for (int64_t j = lo; j < hi; ++j) nc = std::max(nc, chunk_of(p.em_src[j]) + 1);
-        std::vector<int64_t> pos(nc + 1, 0);
-        for (int64_t j = lo; j < hi; ++j) pos[chunk_of(p.em_src[j]) + 1]++;
-        for (int64_t c = 0; c < nc; ++c) pos[c + 1] += pos[c];
-        std::vector<int64_t> start(pos.begin(), pos.end());
-        for (int64_t j = lo; j < hi; ++j) {
-            const int64_t d = lo + pos[chunk_of(p.em_src[j])]++;
-            src[d] = p.em_src[j];
-            row[d] = p.em_row[j];
-        }
-        for (int64_t c = 0; c < nc; ++c) {
-            e.ch_em.push_back(lo + start[c]);
-            e.ch_seg.push_back((int64_t)srow.size());
-            for (int64_t j = lo + start[c]; j < lo + start[c + 1]; ++j)
-                if (j == lo + start[c] || row[j] != row[j - 1]) {
-                    srow.push_back(row[j]);
-                    sstart.push_back(j);
-                }
-        }
+        const int64_t width = std::max(p.n_terms(), k == 0 ? 0 : p.lvl_off[k] - p.lvl_off[k - 1]);
+        base[k + 1] = base[k] + (width + slots - 1) / slots;
     }
-    e.ch_off[D + 1] = (int64_t)e.ch_em.size();
-    e.ch_em.push_back(E);
-    e.ch_seg.push_back((int64_t)srow.size());
-    sstart.push_back(E);
-    upload(src, e.em_src_c);
-    upload(row, e.em_row_c);
-    upload(srow, e.seg_row_c);
-    upload(sstart, e.seg_start_c);
-    e.chunked = true;
+    const int64_t groups = base[D + 1];
+    if (E >= (int64_t)UINT32_MAX - 1 || groups >= (int64_t)UINT32_MAX) return;
+    const bool built = build_order([&] {
+        DevArray<uint64_t> ka(E), kb(E);
+        DevArray<uint32_t> va(E), vb(E), tmp(std::max(dev::sort_scratch(E), dev::scan_scratch(E + 1)) + 1);
+        DevArray<int64_t> d_base((int64_t)base.size()), first(groups + 1);
+        GMR_CUDA(cudaMemcpy(d_base.p, base.data(), base.size() * 8, cudaMemcpyHostToDevice));
+        const int grid = dev::grid_for(E);
+        orders::k_chunk_keys<<<grid, 256>>>(static_cast<const int32_t*>(e.em_src.p), static_cast<const int32_t*>(e.em_row.p),
+                                            E, static_cast<const int64_t*>(e.d_em_off.p),
+                                            static_cast<const int64_t*>(e.d_lvl_off.p), d_base.p, D + 1, slots, ka.p, va.p);
+        uint64_t *k1 = ka.p, *k2 = kb.p;
+        uint32_t *v1 = va.p, *v2 = vb.p;
+        dev::radix_sort(k1, k2, v1, v2, E, bits_for((uint64_t)groups), tmp.p, nullptr);
+        orders::k_group_firsts<<<dev::grid_for(E + 1), 256>>>(k1, E, groups, first.p);
+        e.em_src_c.ensure((size_t)E * 4 + 16);
+        e.em_row_c.ensure((size_t)E * 4 + 16);
+        GMR_CUDA(cudaMemcpyAsync(e.em_src_c.p, v1, (size_t)E * 4, cudaMemcpyDeviceToDevice, nullptr));
+        uint32_t *head = v1, *index = reinterpret_cast<uint32_t*>(k2);  // both are free by now
+        orders::k_chunk_unpack<<<grid, 256>>>(k1, E, static_cast<int32_t*>(e.em_row_c.p), head);
+        dev::exclusive_scan(head, index, E, tmp.p, nullptr);
+        std::vector<int64_t> f((size_t)groups + 1);
+        uint32_t n_seg = 0;
+        GMR_CUDA(cudaMemcpy(f.data(), first.p, f.size() * 8, cudaMemcpyDeviceToHost));
+        GMR_CUDA(cudaMemcpy(&n_seg, index + E, 4, cudaMemcpyDeviceToHost));
+        e.seg_row_c.ensure((size_t)n_seg * 4 + 16);
+        e.seg_start_c.ensure(((size_t)n_seg + 1) * 8 + 16);
+        orders::k_chunk_segments<<<dev::grid_for(E + 1), 256>>>(k1, head, index, E, static_cast<int32_t*>(e.seg_row_c.p),
+                                                                static_cast<int64_t*>(e.seg_start_c.p));
+        e.ch_off.assign(D + 2, 0);
+        e.ch_em.clear();
+        for (int k = 0; k <= D; ++k) {  // a level's chunks, up to the last one that emits
+            e.ch_off[k] = (int64_t)e.ch_em.size();
+            int64_t g1 = base[k + 1];
+            while (g1 > base[k] && f[g1] == f[g1 - 1]) --g1;
+            for (int64_t g = base[k]; g < g1; ++g) e.ch_em.push_back(f[g]);
+        }
+        e.ch_off[D + 1] = (int64_t)e.ch_em.size();
+        e.ch_em.push_back(E);
+        e.ch_seg.assign(e.ch_em.size(), 0);
+        DevArray<int64_t> at((int64_t)e.ch_em.size());
+        GMR_CUDA(cudaMemcpy(at.p, e.ch_em.data(), e.ch_em.size() * 8, cudaMemcpyHostToDevice));
+        orders::k_pick<<<dev::grid_for((int64_t)e.ch_em.size()), 256>>>(index, at.p, (int64_t)e.ch_em.size(), at.p);
+        GMR_CUDA(cudaGetLastError());
+        GMR_CUDA(cudaMemcpy(e.ch_seg.data(), at.p, e.ch_seg.size() * 8, cudaMemcpyDeviceToHost));
+        e.chunked = true;
+    });
+    if (!built) {
+        for (auto* b : {&e.em_src_c, &e.em_row_c, &e.seg_row_c, &e.seg_start_c}) b->release();
+        e.ch_off.clear();
+        e.ch_em.clear();
+        e.ch_seg.clear();
+    }
 }
 
 // Direct terminal emissions pay off when the terminal table is much larger
@@ -1950,33 +1988,44 @@ static void build_direct_terms(const gmr_plan& p, gmr_engine& e) {
     upload(list, e.rule_terms);
 }
 
-// Push lists (gmr_engine::pe_*): a counting sort of the emissions of levels
-// 1..depth by source slot.  The plan orders a level's emissions by (row,
-// source), so each slot's rows come out ascending.  Offsets are int32: a
-// plan with 2^31 or more such emissions gets no push lists.
+// Push lists (gmr_engine::pe_*): the emissions of levels 1..depth stably sorted
+// by source slot.  The plan orders a level's emissions by (row, source), so
+// each slot's rows come out ascending.  Offsets are int32: a plan with 2^31 or
+// more such emissions gets no push lists.
 static void build_push_lists(const gmr_plan& p, gmr_engine& e) {
     const int D = p.depth;
     e.push_ok.assign(D + 2, 0);
     if (D < 1) return;
-    const int64_t E0 = p.em_off[1], E1 = p.em_off[D + 1];
-    if (E1 - E0 >= (int64_t)INT32_MAX || p.n_ops() >= (int64_t)INT32_MAX) return;
-    std::vector<int32_t> off((size_t)p.n_ops() + 1, 0);
-    for (int k = 1; k <= D; ++k) {
-        bool ok = true;
-        for (int64_t j = p.em_off[k]; j < p.em_off[k + 1] && ok; ++j)
-            ok = p.em_src[j] >= p.lvl_off[k - 1] && p.em_src[j] < p.lvl_off[k];
-        e.push_ok[k] = ok;
-        if (!ok) continue;
-        for (int64_t j = p.em_off[k]; j < p.em_off[k + 1]; ++j) off[(size_t)p.em_src[j] + 1]++;
+    const int64_t E0 = p.em_off[1], n = p.em_off[D + 1] - E0, n_ops = p.n_ops();
+    if (n >= (int64_t)INT32_MAX || n_ops >= (int64_t)INT32_MAX) return;
+    const bool built = build_order([&] {
+        DevArray<uint8_t> mixed(D + 2);
+        GMR_CUDA(cudaMemsetAsync(mixed.p, 0, (size_t)D + 2, nullptr));
+        const int32_t *src = static_cast<const int32_t*>(e.em_src.p), *row = static_cast<const int32_t*>(e.em_row.p);
+        const int64_t *em_off = static_cast<const int64_t*>(e.d_em_off.p), *lvl_off = static_cast<const int64_t*>(e.d_lvl_off.p);
+        DevArray<uint64_t> ka(n), kb(n);
+        DevArray<uint32_t> va(n), vb(n), tmp(dev::sort_scratch(n) + 1);
+        e.pe_off.ensure(((size_t)n_ops + 1) * 4 + 16);
+        e.pe_row.ensure((size_t)std::max<int64_t>(n, 1) * 4 + 16);
+        uint64_t *k1 = ka.p, *k2 = kb.p;
+        uint32_t *v1 = va.p, *v2 = vb.p;
+        const int grid = dev::grid_for(n);
+        if (n) {
+            orders::k_mixed_levels<<<grid, 256>>>(src, E0, E0 + n, em_off, lvl_off, D + 1, mixed.p);
+            orders::k_push_keys<<<grid, 256>>>(src, row, E0, n, em_off, D + 1, mixed.p, n_ops, k1, v1);
+            dev::radix_sort(k1, k2, v1, v2, n, bits_for((uint64_t)n_ops), tmp.p, nullptr);
+            GMR_CUDA(cudaMemcpyAsync(e.pe_row.p, v1, (size_t)n * 4, cudaMemcpyDeviceToDevice, nullptr));
+        }
+        orders::k_group_firsts<<<dev::grid_for(n + 1), 256>>>(k1, n, n_ops, static_cast<int32_t*>(e.pe_off.p));
+        GMR_CUDA(cudaGetLastError());
+        std::vector<uint8_t> m((size_t)D + 2);
+        GMR_CUDA(cudaMemcpy(m.data(), mixed.p, m.size(), cudaMemcpyDeviceToHost));
+        for (int k = 1; k <= D; ++k) e.push_ok[k] = !m[k];
+    });
+    if (!built) {
+        e.pe_off.release();
+        e.pe_row.release();
     }
-    for (size_t s = 0; s + 1 < off.size(); ++s) off[s + 1] += off[s];
-    std::vector<int32_t> row((size_t)std::max<int32_t>(off.back(), 1)), fill(off.begin(), off.end() - 1);
-    for (int k = 1; k <= D; ++k) {
-        if (!e.push_ok[k]) continue;
-        for (int64_t j = p.em_off[k]; j < p.em_off[k + 1]; ++j) row[(size_t)fill[(size_t)p.em_src[j]]++] = p.em_row[j];
-    }
-    upload(off, e.pe_off);
-    upload(row, e.pe_row);
 }
 
 // The (chunk, row) order of the one-word fold (word_fold.cuh), sorted on the
@@ -1990,12 +2039,9 @@ static void build_word_fold(gmr_engine& e) {
     if (e.direct_terms || e.n_ops == 0 || E < kWordMinEmissions || E >= (int64_t)UINT32_MAX - 1 ||
         (double)E < kWordMinPerRow * (double)chunks * (double)e.rows || chunks * blks > (1 << 20))
         return;
-    int row_bits = 16;  // at least the 16 bits an entry keeps
-    while ((1ll << row_bits) < e.rows) ++row_bits;
-    int chunk_bits = 1;
-    while ((1ll << chunk_bits) < chunks) ++chunk_bits;
+    const int row_bits = std::max(16, bits_for((uint64_t)e.rows));  // at least the 16 bits an entry keeps
     const int n_seg = (int)(chunks * blks);
-    try {
+    const bool built = build_order([&] {
         DevArray<uint64_t> ka(E), kb(E);
         DevArray<uint32_t> tmp(dev::sort_scratch(E) + 1), first(n_seg + 1);
         k_word_keys<<<dev::grid_for(E), 256>>>(static_cast<const int32_t*>(e.em_src.p),
@@ -2003,7 +2049,7 @@ static void build_word_fold(gmr_engine& e) {
                                                row_bits, ka.p);
         uint64_t *k1 = ka.p, *k2 = kb.p;
         uint32_t *v1 = nullptr, *v2 = nullptr;
-        dev::radix_sort(k1, k2, v1, v2, E, row_bits + chunk_bits, tmp.p, nullptr);
+        dev::radix_sort(k1, k2, v1, v2, E, row_bits + bits_for((uint64_t)chunks), tmp.p, nullptr);
         k_word_segments<<<dev::grid_for(n_seg + 1), 256>>>(k1, E, row_bits, (int)blks, n_seg, first.p);
         GMR_CUDA(cudaGetLastError());
         std::vector<uint32_t> f((size_t)n_seg + 1), seg((size_t)n_seg + 1, 0);
@@ -2019,8 +2065,8 @@ static void build_word_fold(gmr_engine& e) {
                                                 static_cast<uint32_t*>(e.word_entries.p));
         GMR_CUDA(cudaGetLastError());
         GMR_CUDA(cudaStreamSynchronize(nullptr));
-    } catch (const Error& err) {
-        if (err.code != GMR_ERR_OOM) throw;
+    });
+    if (!built) {
         e.word_entries.release();
         e.word_seg.release();
         e.word_parts.release();

@@ -104,22 +104,37 @@ __global__ void k_group_fill(const uint64_t* __restrict__ key, const uint32_t* _
     }
 }
 
-// Ranking key of each distinct pair: (count desc, key asc) for candidates
-// (count >= 2), all ones otherwise.  Distinct pairs are in ascending key order,
-// so u stands for the key.
-__global__ void k_rank_keys(const uint32_t* __restrict__ ustart, const uint32_t* __restrict__ cpre, int64_t nu,
-                            int64_t nv, int bu, uint64_t* rkey, uint32_t* rval, unsigned long long* n_cand) {
-    unsigned long long nc = 0;
+// Count of each distinct pair; stats[0] += candidates (count >= 2), stats[1] =
+// the largest count.
+__global__ void k_pair_counts(const uint32_t* __restrict__ ustart, const uint32_t* __restrict__ cpre, int64_t nu,
+                              int64_t nv, uint32_t* count, unsigned long long* stats) {
+    unsigned long long nc = 0, mx = 0;
     GRID_STRIDE(u, nu) {
         const uint32_t a = ustart[u], b = u + 1 < nu ? ustart[u + 1] : (uint32_t)nv;
         const uint32_t c = cpre[b] - cpre[a];
-        const bool cand = c >= 2;
-        rkey[u] = cand ? (((uint64_t)(0x80000000u - c) << bu) | (uint64_t)u) : ~0ull;
-        rval[u] = (uint32_t)u;
-        nc += cand;
+        count[u] = c;
+        nc += c >= 2;
+        mx = max(mx, (unsigned long long)c);
     }
-    for (int o = 16; o; o >>= 1) nc += __shfl_xor_sync(0xffffffffu, nc, o);
-    if ((threadIdx.x & 31) == 0 && nc) atomicAdd(n_cand, nc);
+    for (int o = 16; o; o >>= 1) {
+        nc += __shfl_xor_sync(0xffffffffu, nc, o);
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (nc) atomicAdd(&stats[0], nc);
+        atomicMax(&stats[1], mx);
+    }
+}
+
+// Ranking key of each distinct pair: count descending, no candidate (count < 2)
+// last.  Distinct pairs are in ascending key order and the sort is stable, so
+// equal counts stay in key order: the key needs the counts' bits alone, one or
+// two digits in most rounds, where (count, key) packed took seven.
+__global__ void k_rank_keys(const uint32_t* __restrict__ count, int64_t nu, uint32_t most, uint64_t* rkey, uint32_t* rval) {
+    GRID_STRIDE(u, nu) {
+        rkey[u] = count[u] >= 2 ? most - count[u] : most - 1;
+        rval[u] = (uint32_t)u;
+    }
 }
 
 __global__ void k_fill_u32(uint32_t* a, int64_t n, uint32_t v) {
@@ -227,6 +242,13 @@ T read1(const T* d, cudaStream_t st) {
         GMR_CUDA(cudaGetLastError());                                   \
     } while (0)
 
+// At least n elements, with room to spare when it has to grow (its contents
+// are not kept).
+template <class T>
+void reserve(DevArray<T>& a, int64_t n) {
+    if (a.n < n || !a.p) a.alloc(n + n / 4 + 1);
+}
+
 struct Stream {
     cudaStream_t s = nullptr;
     Stream() { GMR_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking)); }
@@ -266,7 +288,11 @@ extern "C" int gmr_repair_compress_device(const gmr_csrv* m, int device, gmr_gra
         DevArray<uint32_t> tmp(std::max(dev::sort_scratch(cap), dev::scan_scratch(cap + 1)) + 1);
         DevArray<unsigned long long> cnt(4);
         std::vector<int32_t> rules;           // host copy, appended per round
-        DevArray<int32_t> new_rules(0);
+        // buffers of the rounds' candidates, kept from round to round: their sizes
+        // are known late, and allocating them in every round took half of a late one
+        DevArray<uint64_t> rk, rk2;
+        DevArray<uint32_t> rv, rv2, rank_of, acc;
+        DevArray<int32_t> new_rules;
 
         for (int round = 0; round < 100000 && n > 1; ++round) {
             auto t0 = std::chrono::steady_clock::now();
@@ -297,16 +323,22 @@ extern "C" int gmr_repair_compress_device(const gmr_csrv* m, int device, gmr_gra
             uint32_t* ustart = p2;
             LAUNCH(k_group_fill, nv, k1, w1.p, w2.p, nv, ustart, ukey);
             // (3) rank the candidates
-            DevArray<uint64_t> rk(nu), rk2(nu);
-            DevArray<uint32_t> rv(nu), rv2(nu), rank_of(nu);
-            const int bu = bits_of((uint64_t)nu);
-            LAUNCH(k_rank_keys, nu, ustart, w3.p, nu, nv, bu, rk.p, rv.p, cnt.p + 1);
-            const int64_t ncand = (int64_t)read1(cnt.p + 1, st);
+            reserve(rk, nu);
+            reserve(rk2, nu);
+            reserve(rv, nu);
+            reserve(rv2, nu);
+            reserve(rank_of, nu);
+            LAUNCH(k_pair_counts, nu, ustart, w3.p, nu, nv, rank_of.p, cnt.p);
+            unsigned long long stats[2];
+            GMR_CUDA(cudaMemcpyAsync(stats, cnt.p, sizeof(stats), cudaMemcpyDeviceToHost, st));
+            GMR_CUDA(cudaStreamSynchronize(st));
+            const int64_t ncand = (int64_t)stats[0];
             if (ncand == 0) break;
             if (ncand + maxsym > INT32_MAX) throw Error(GMR_ERR_RANGE, "grammar exceeds the int32 symbol space");
+            LAUNCH(k_rank_keys, nu, rank_of.p, nu, (uint32_t)stats[1], rk.p, rv.p);
             uint64_t *r1 = rk.p, *r2 = rk2.p;
             uint32_t *q1 = rv.p, *q2 = rv2.p;
-            dev::radix_sort(r1, r2, q1, q2, nu, 32 + bu, tmp.p, st);
+            dev::radix_sort(r1, r2, q1, q2, nu, bits_of(stats[1] - 1), tmp.p, st);
             LAUNCH(k_fill_u32, nu, rank_of.p, nu, NONE);
             LAUNCH(k_rank_of, ncand, q1, ncand, rank_of.p);
             // rank at every position (w3 is free again after this)
@@ -322,13 +354,13 @@ extern "C" int gmr_repair_compress_device(const gmr_csrv* m, int device, gmr_gra
             uint32_t* f = w1.p;
             LAUNCH(k_chosen_sorted, nv, p1, chosen.p, nv, f);
             dev::exclusive_scan(f, f, nv, tmp.p, st);
-            DevArray<uint32_t> acc(ncand + 1);
+            reserve(acc, ncand + 1);
             LAUNCH(k_accept, ncand, q1, ustart, f, ncand, nu, nv, acc.p);
             uint32_t* apre = w2.p;  // group indices no longer needed
             dev::exclusive_scan(acc.p, apre, ncand, tmp.p, st);
             const int64_t nacc = (int64_t)read1(apre + ncand, st);
             if (nacc == 0) break;
-            new_rules.alloc(2 * nacc);
+            reserve(new_rules, 2 * nacc);
             LAUNCH(k_new_rules, ncand, q1, ukey, acc.p, apre, ncand, b, new_rules.p);
             const size_t r0 = rules.size();
             rules.resize(r0 + 2 * (size_t)nacc);

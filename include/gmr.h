@@ -315,7 +315,8 @@ int gmr_engine_time_launches(gmr_engine* e, int semiring, const void* dX, void* 
  * table is used by GMR_VARIANT_AUTO multiplies of that (semiring, B).
  * With one 4-byte word per value (B = 1, or up to 32 Boolean right-hand sides)
  * and enough emissions the engine folds every level's emissions in one launch
- * after the rules, and a table has nothing to choose.
+ * after the rules, and a table has nothing to choose; with one lane per value
+ * (1, 2 or 4 words) e = 3 and 4 run the segmented fold, which is faster there.
  * Adding GMR_LEVEL_PUSH to slot k's entry (1 <= k <= depth) makes the rules of
  * level k push their values into the rows that emit them as soon as they are
  * computed (vector reductions into Y, which stays in L2), so launch k+1
