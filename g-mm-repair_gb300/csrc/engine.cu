@@ -1006,6 +1006,14 @@ struct Launch {
     }
 };
 
+// A list for k_word_fold on the device.
+struct WordList {
+    DevBuf entries, seg;
+    int segs = 0, blks = 0;
+    int64_t groups = 0;
+    bool ready = false;
+};
+
 struct GraphEntry {
     cudaGraphExec_t exec = nullptr;
     Launch lc{};
@@ -1050,12 +1058,14 @@ struct gmr_engine {
     // level k has a slot of level k as its source, so level k can push.
     gmr::DevBuf pe_off, pe_row;
     std::vector<uint8_t> push_ok;
-    // One-word fold (word_fold.cuh): the emissions in (chunk, row) order.
-    gmr::DevBuf word_entries, word_seg;
+    // One-word folds (word_fold.cuh): the emissions in (chunk, row) order, and
+    // for the left product in (chunk of rows, target) order.
+    gmr::WordList word, left_word;
     gmr::DevBuf word_parts;  // scratch: the copies of Y that chunks add into ((+,x) only)
-    int word_segs = 0, word_blks = 0, word_copies = 1;
-    int64_t word_groups = 0;
-    bool word_ready = false;
+    int word_copies = 1;
+    // Left product at one word per value: the parent edges alone, by level.
+    gmr::DevBuf lp_src, lp_tgt;
+    std::vector<int64_t> lp_first, lp_count;
     // Left product (y = x^T M): flat edge lists uploaded by gmr_engine_enable_left.
     gmr::DevBuf le_src, le_tgt, le_split, tcol_off, tcol_q;
     std::vector<int64_t> le_off, le_first;  // the plan's offsets; where each range starts on the device
@@ -1082,7 +1092,8 @@ struct gmr_engine {
         return {&ops, &op_c, &em_src, &em_row, &seg_row, &seg_start, &term_val, &term_col, &V,
                 &d_lvl_off, &d_em_off, &d_seg_off, &sync, &em_src_c, &em_row_c, &seg_row_c, &seg_start_c,
                 &le_src, &le_tgt, &le_split, &tcol_off, &tcol_q, &em_tcode, &rule_terms, &ops_direct,
-                &pe_off, &pe_row, &word_entries, &word_seg, &word_parts};
+                &pe_off, &pe_row, &word.entries, &word.seg, &word_parts, &left_word.entries, &left_word.seg,
+                &lp_src, &lp_tgt};
     }
 };
 
@@ -1200,15 +1211,19 @@ static void launch_level(int emit, dim3 grid, cudaStream_t st, bool pdl, const S
 template <class S>
 static int word_copies(const gmr_engine* e) { return std::is_same<S, SPlus>::value ? e->word_copies : 1; }
 
+static void set_word_list(WordFoldArgs& w, const WordList& l) {
+    w.entries = static_cast<const uint4*>(l.entries.p);
+    w.seg = static_cast<const uint32_t*>(l.seg.p);
+    w.n_seg = l.segs;
+    w.n_blk = l.blks;
+    w.n_groups = l.groups;
+}
+
 // The one-launch fold of all emissions (word_fold.cuh) into Y ([copies][rows]).
 template <class S>
 static void launch_word_fold(const gmr_engine* e, void* Y, int copies, cudaStream_t st, bool pdl) {
     WordFoldArgs w{};
-    w.entries = static_cast<const uint4*>(e->word_entries.p);
-    w.seg = static_cast<const uint32_t*>(e->word_seg.p);
-    w.n_seg = e->word_segs;
-    w.n_blk = e->word_blks;
-    w.n_groups = e->word_groups;
+    set_word_list(w, e->word);
     w.T = e->T.p;
     w.arena = e->arena.p;
     w.n_terms = e->n_terms;
@@ -1731,7 +1746,7 @@ static Launch resolve_launch(gmr_engine* e, int semiring, int B, const void* X, 
     else if (lc.Bt % 2 == 0 && lc.Bw % 2 == 0 && aligned(8)) lc.VEC = 2;
     else lc.VEC = 1;
     lc.G = lc.Bt / lc.VEC;
-    lc.word = e->word_ready && lc.Bw == 1 && max_vec >= 8 && lc.push_mode == GMR_PUSH_AUTO &&
+    lc.word = e->word.ready && lc.Bw == 1 && max_vec >= 8 && lc.push_mode == GMR_PUSH_AUTO &&
               (lc.variant == GMR_VARIANT_GRAPH || lc.variant == GMR_VARIANT_FUSED) &&
               !(cfg && (cfg->emit_mode || cfg->ops_per_cta > 0)) &&
               (semiring != GMR_PLUS_TIMES || e->n_em >= kWordMinEmissionsPlus);
@@ -2028,25 +2043,25 @@ static void build_push_lists(const gmr_plan& p, gmr_engine& e) {
     }
 }
 
-// The (chunk, row) order of the one-word fold (word_fold.cuh), sorted on the
-// GPU from the uploaded emissions.  Not built where it does not pay: graphs
-// with direct terminals (their terminals are no table), too few emissions, or
-// runs too short (kWordMinPerRow).  Without the memory for it the engine keeps
-// the per-level folds.
-static void build_word_fold(gmr_engine& e) {
-    const int64_t E = e.n_em, total = word_t_span(e.n_terms) + e.n_ops;
-    const int64_t chunks = (total + kWordChunk - 1) / kWordChunk, blks = ((int64_t)e.rows + 65535) / 65536;
-    if (e.direct_terms || e.n_ops == 0 || E < kWordMinEmissions || E >= (int64_t)UINT32_MAX - 1 ||
-        (double)E < kWordMinPerRow * (double)chunks * (double)e.rows || chunks * blks > (1 << 20))
+// A (chunk, target) order of the emissions for k_word_fold, sorted on the GPU
+// from the uploaded ones: of `values` values into `targets` targets, the left
+// product's when left_terms >= 0 (its terminals' first target).  Not built where
+// it does not pay: graphs with direct terminals (their terminals are no table),
+// too few emissions, runs too short (kWordMinPerRow).
+static void build_word_list(gmr_engine& e, WordList& l, int64_t values, int64_t targets, int64_t left_terms) {
+    const int64_t E = e.n_em, chunks = (values + kWordChunk - 1) / kWordChunk, blks = (targets + 65535) / 65536;
+    if (l.ready || e.direct_terms || e.n_ops == 0 || E < kWordMinEmissions || E >= (int64_t)UINT32_MAX - 1 ||
+        (double)E < kWordMinPerRow * (double)chunks * (double)targets || chunks * blks > (1 << 20))
         return;
-    const int row_bits = std::max(16, bits_for((uint64_t)e.rows));  // at least the 16 bits an entry keeps
+    const int row_bits = std::max(16, bits_for((uint64_t)targets));  // at least the 16 bits an entry keeps
     const int n_seg = (int)(chunks * blks);
+    const uint32_t zero_at = (uint32_t)std::min<int64_t>(values, kWordChunk);
     const bool built = build_order([&] {
         DevArray<uint64_t> ka(E), kb(E);
         DevArray<uint32_t> tmp(dev::sort_scratch(E) + 1), first(n_seg + 1);
         k_word_keys<<<dev::grid_for(E), 256>>>(static_cast<const int32_t*>(e.em_src.p),
                                                static_cast<const int32_t*>(e.em_row.p), E, word_t_span(e.n_terms),
-                                               row_bits, ka.p);
+                                               row_bits, left_terms >= 0, left_terms, ka.p);
         uint64_t *k1 = ka.p, *k2 = kb.p;
         uint32_t *v1 = nullptr, *v2 = nullptr;
         dev::radix_sort(k1, k2, v1, v2, E, row_bits + bits_for((uint64_t)chunks), tmp.p, nullptr);
@@ -2055,29 +2070,37 @@ static void build_word_fold(gmr_engine& e) {
         std::vector<uint32_t> f((size_t)n_seg + 1), seg((size_t)n_seg + 1, 0);
         GMR_CUDA(cudaMemcpy(f.data(), first.p, f.size() * 4, cudaMemcpyDeviceToHost));
         for (int i = 0; i < n_seg; ++i) seg[i + 1] = seg[i] + (f[i + 1] - f[i] + kWordGroup - 1) / kWordGroup;
-        e.word_groups = seg[n_seg];
-        upload(seg, e.word_seg);
-        e.word_entries.ensure((size_t)e.word_groups * kWordGroup * 4);
-        e.word_copies = (int)std::min<int64_t>(kWordMaxCopies, (chunks + kWordChunksPerCopy - 1) / kWordChunksPerCopy);
-        if (e.word_copies > 1) e.word_parts.ensure((size_t)e.rows * e.word_copies * 4);
-        k_word_entries<<<e.sm_count * 8, 256>>>(k1, first.p, static_cast<const uint32_t*>(e.word_seg.p), n_seg,
-                                                e.word_groups, (uint32_t)word_zero_at(e.n_terms, e.n_ops),
-                                                static_cast<uint32_t*>(e.word_entries.p));
+        l.groups = seg[n_seg];
+        upload(seg, l.seg);
+        l.entries.ensure((size_t)l.groups * kWordGroup * 4);
+        k_word_entries<<<e.sm_count * 8, 256>>>(k1, first.p, static_cast<const uint32_t*>(l.seg.p), n_seg, l.groups, zero_at,
+                                                static_cast<uint32_t*>(l.entries.p));
         GMR_CUDA(cudaGetLastError());
         GMR_CUDA(cudaStreamSynchronize(nullptr));
     });
     if (!built) {
-        e.word_entries.release();
-        e.word_seg.release();
-        e.word_parts.release();
+        l.entries.release();
+        l.seg.release();
         return;
     }
     for (auto* k : {(const void*)k_word_fold<SPlus>, (const void*)k_word_fold<SBool>, (const void*)k_word_fold<STrop>})
         GMR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (kWordChunk + 1) * 4));
-    e.word_segs = n_seg;
-    e.word_blks = (int)blks;
-    e.word_ready = true;
+    l.segs = n_seg;
+    l.blks = (int)blks;
+    l.ready = true;
 }
+
+static void build_word_fold(gmr_engine& e) {
+    const int64_t values = word_t_span(e.n_terms) + e.n_ops, chunks = (values + kWordChunk - 1) / kWordChunk;
+    build_word_list(e, e.word, values, e.rows, -1);
+    e.word_copies = (int)std::min<int64_t>(kWordMaxCopies, (chunks + kWordChunksPerCopy - 1) / kWordChunksPerCopy);
+    if (!e.word.ready || e.word_copies == 1) return;
+    if (!build_order([&] { e.word_parts.ensure((size_t)e.rows * e.word_copies * 4); })) e.word_copies = 1;
+}
+
+// Where the terminals' targets start in the left product's list: a whole number
+// of blocks of 65,536.
+static int64_t left_word_terms(const gmr_engine* e) { return (e->n_ops + 65535) / 65536 * 65536; }
 
 extern "C" int gmr_engine_create(const gmr_plan* p, int device, gmr_engine** out) {
     return guarded([&] {
@@ -2525,9 +2548,12 @@ extern "C" void gmr_engine_free(gmr_engine* e) {
 // words per value a warp folds 128 consecutive edges (fold_runs) instead of
 // each lane walking 16 of its own.
 // The launches follow each other by programmatic dependent launch in a cached
-// graph.  Measured on 50,000 x 5,000 (20 M edges), before -> now: B = 1 342 ->
-// 173 us, B = 32 698 -> 492 us; 3,149 x 575, B = 2 137 -> 59 us; 29,229 x 2,388,
-// B = 10 330 -> 204 us.
+// graph.  At one word per value the rows' edges, three quarters of all, are
+// folded at once out of shared memory (k_word_fold with x as its values), and
+// only the parents' go level by level.
+// Measured on 50,000 x 5,000 (20 M edges), before -> now: B = 1 342 -> 173 us, 157
+// with the rows' edges at once, B = 32 698 -> 454 us; 3,149 x 575, B = 2 137 -> 57
+// us; 29,229 x 2,388, B = 10 330 -> 220 us.
 namespace gmr {
 
 struct LeftArgs {
@@ -2652,7 +2678,9 @@ static int left_chunk(int64_t n) {
     return n <= (1 << 16) ? 4 : n <= (1 << 18) ? 8 : (int)kLeftChunk;
 }
 
-template <class S, int VEC>
+// ADD: every target already holds a value (the rows' part, from k_word_fold),
+// and sums are added to it.
+template <class S, int VEC, bool ADD>
 __global__ void __launch_bounds__(256) k_left_fold_warp(LeftArgs a) {
     using T = typename S::T;
     dependents_may_launch();
@@ -2683,9 +2711,28 @@ __global__ void __launch_bounds__(256) k_left_fold_warp(LeftArgs a) {
         const bool cut_first = e0 > 0 && __ldg(tgt + e0 - 1) == tfirst;
         const bool cut_last = e1 < a.count && __ldg(tgt + e1) == tlast;
         fold_runs<S, VEC>(u, v, lane, [&](int32_t t, const Vec<T, VEC>& sum) {
-            if (t != kNone) left_flush<S, VEC>(a, t, 0, !((cut_first && t == tfirst) || (cut_last && t == tlast)), sum);
+            if (t == kNone) return;
+            const bool whole = !((cut_first && t == tfirst) || (cut_last && t == tlast));
+            if constexpr (ADD) {
+                T* p = static_cast<T*>(a.terminals ? a.tdown : a.down) + (int64_t)t * VEC;
+                if (whole) vstore<T, VEC>(p, voplus<S, VEC>(vload_rw<T, VEC>(p), sum));
+                else vred<S, VEC>(p, sum);
+            } else {
+                left_flush<S, VEC>(a, t, 0, whole, sum);
+            }
         });
     }
+}
+
+// Every down value to the semiring zero (n_ops rules, then count terminals).
+template <class S>
+__global__ void __launch_bounds__(256) k_left_clear(LeftArgs a) {
+    using T = typename S::T;
+    dependents_may_launch();
+    wait_for_previous_kernel();
+    const int64_t n = a.n_ops + a.count;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256)
+        *(i < a.n_ops ? static_cast<T*>(a.down) + i : static_cast<T*>(a.tdown) + (i - a.n_ops)) = S::zero();
 }
 
 template <class S, int VEC, int GLOG>
@@ -2742,6 +2789,36 @@ static void left_chain_t(gmr_engine* e, const Launch& lc, const void* X, void* Y
         ++launches;
     };
     const int D = e->depth;
+    if constexpr (VEC == 1 && GLOG == 0) {
+        if (lc.word) {  // all rows' parts in one launch out of shared memory, then the parents level by level
+            a.count = e->n_terms;
+            launch(k_left_clear<S>, blocks(e->n_ops + e->n_terms), a);
+            WordFoldArgs w{};
+            set_word_list(w, e->left_word);
+            w.T = w.arena = X;
+            w.n_ops = e->rows;
+            w.zero_at = (int)std::min<int64_t>(e->rows, kWordChunk);
+            w.Y = e->arena.p;
+            w.copies = 1;
+            w.Yterm = e->T.p;
+            w.term_blk = (int)(left_word_terms(e) >> 16);
+            launch_kernel_n(k_word_fold<S>, dim3(e->sm_count), kWordThreads, (size_t)(w.zero_at + 1) * 4, st, pdl, w);
+            ++launches;
+            a.src = static_cast<const int32_t*>(e->lp_src.p);
+            a.tgt = static_cast<const int32_t*>(e->lp_tgt.p);
+            for (int j = D; j >= 0; --j) {
+                const int k = j ? j : D + 1;
+                a.first = e->lp_first[k - 1];
+                a.count = e->lp_count[k];
+                a.terminals = k == D + 1;
+                if (a.count) launch(k_left_fold_warp<S, 1, true>, blocks((a.count + kLeftGroup - 1) / kLeftGroup * 32), a);
+            }
+            a.first = 0;
+            a.count = e->cols;
+            launch(k_left_columns<S, 1, 0>, blocks(e->cols), a);
+            return;
+        }
+    }
     if (lc.padded)
         launch(k_restride<T>, blocks((int64_t)e->rows * lc.Bp), static_cast<const T*>(X), static_cast<T*>(e->padX.p),
                (int64_t)e->rows, lc.Bw, lc.Bw, lc.Bp, T(0));
@@ -2755,7 +2832,7 @@ static void left_chain_t(gmr_engine* e, const Launch& lc, const void* X, void* Y
         a.chunk = left_chunk(a.count);
         if (a.count == 0) continue;
         if constexpr (GLOG == 0 && VEC <= 2)
-            launch(k_left_fold_warp<S, VEC>, blocks((a.count + kLeftGroup - 1) / kLeftGroup * 32), a);
+            launch(k_left_fold_warp<S, VEC, false>, blocks((a.count + kLeftGroup - 1) / kLeftGroup * 32), a);
         else
             launch(k_left_fold<S, VEC, GLOG>, blocks((a.count + a.chunk - 1) / a.chunk * G), a);
     }
@@ -2810,6 +2887,7 @@ static Launch resolve_left(gmr_engine* e, int semiring, int B, const void* X, vo
     else if (lc.Bp == 2 && aligned(8)) lc.VEC = 2;
     else lc.VEC = 1;
     lc.G = lc.Bp / lc.VEC;
+    lc.word = lc.Bw == 1 && e->left_word.ready && aligned(16);
     return lc;
 }
 
@@ -2840,6 +2918,27 @@ extern "C" int gmr_engine_enable_left(gmr_engine* e, gmr_plan* p) {
                                     cudaMemcpyHostToDevice));
             }
             e->le_first = std::move(first);
+        }
+        // the rows' edges once more for the one-word fold, and the parents' alone
+        build_word_list(*e, e->left_word, e->rows, left_word_terms(e) + e->n_terms, left_word_terms(e));
+        if (e->left_word.ready) {
+            const int D = e->depth;
+            std::vector<int32_t> src, tgt;
+            e->lp_first.assign((size_t)D + 2, 0);
+            e->lp_count.assign((size_t)D + 2, 0);
+            for (int k = 1; k <= D + 1; ++k) {
+                src.resize((src.size() + 3) & ~(size_t)3, 0);
+                tgt.resize(src.size(), 0);
+                e->lp_first[k - 1] = (int64_t)src.size();
+                for (int64_t i = p->le_off[k - 1]; i < p->le_off[k]; ++i)
+                    if ((int64_t)p->le_src[i] < e->n_ops) {
+                        src.push_back(p->le_src[i]);
+                        tgt.push_back(p->le_tgt[i]);
+                    }
+                e->lp_count[k] = (int64_t)src.size() - e->lp_first[k - 1];
+            }
+            upload(src, e->lp_src);
+            upload(tgt, e->lp_tgt);
         }
         // targets whose edges straddle the chunks used here (the plan's list is for kLeftChunk throughout)
         std::vector<int32_t> split;

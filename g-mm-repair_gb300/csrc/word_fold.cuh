@@ -66,6 +66,10 @@ struct WordFoldArgs {
     void* Y;                   // [copies][rows]: chunk c adds into copy c % copies
     int64_t rows;
     int copies;
+    // Left product: the targets are the rules' and then, from block of rows
+    // term_blk on, the terminals' down values.  nullptr: rows of Y throughout.
+    void* Yterm;
+    int term_blk;
 };
 
 // Chunk `chunk` of the value space into shared memory, 16 bytes per load (both
@@ -185,7 +189,9 @@ __global__ void __launch_bounds__(kWordThreads, 1) k_word_fold(WordFoldArgs a) {
         const int64_t to = min((int64_t)__ldg(a.seg + s + 1), end);
         if (to <= at) continue;
         const int chunk = s / a.n_blk;
-        T* Y = static_cast<T*>(a.Y) + (chunk % a.copies) * a.rows + ((int64_t)(s - chunk * a.n_blk) << 16);
+        const int blk = s - chunk * a.n_blk;
+        T* Y = a.Yterm && blk >= a.term_blk ? static_cast<T*>(a.Yterm) + ((int64_t)(blk - a.term_blk) << 16)
+                                            : static_cast<T*>(a.Y) + (chunk % a.copies) * a.rows + ((int64_t)blk << 16);
         if (chunk != loaded) {
             __syncthreads();  // the chunk before is no longer read
             load_word_chunk<T>(a, chunk, vals);
@@ -218,15 +224,17 @@ __global__ void __launch_bounds__(256) k_word_sum(const typename S::T* __restric
 }
 
 // Sort keys of the emissions: source in chunk << 48 | chunk << row_bits | row,
-// to be sorted by the bits below 48.
+// to be sorted by the bits below 48.  left: rows are gathered (the value space
+// is x) and the targets are rules, then terminals from left_terms on.
 static __global__ void __launch_bounds__(256) k_word_keys(const int32_t* __restrict__ src, const int32_t* __restrict__ row,
-                                                          int64_t n, int64_t t_span, int row_bits,
-                                                          uint64_t* __restrict__ key) {
+                                                          int64_t n, int64_t t_span, int row_bits, bool left,
+                                                          int64_t left_terms, uint64_t* __restrict__ key) {
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
         const int32_t c = src[i];
-        const int64_t v = c >= 0 ? t_span + c : -(int64_t)c - 1;
+        const int64_t v = left ? (int64_t)row[i] : c >= 0 ? t_span + c : -(int64_t)c - 1;
+        const int64_t to = !left ? (int64_t)row[i] : c >= 0 ? (int64_t)c : left_terms - (int64_t)c - 1;
         const int64_t chunk = v / kWordChunk;
-        key[i] = (uint64_t)(v - chunk * kWordChunk) << 48 | (uint64_t)chunk << row_bits | (uint32_t)row[i];
+        key[i] = (uint64_t)(v - chunk * kWordChunk) << 48 | (uint64_t)chunk << row_bits | (uint64_t)to;
     }
 }
 

@@ -53,3 +53,45 @@ def test_word_fold(name, sr):
         np.testing.assert_array_equal(a, b)
     else:
         assert np.abs(a - b).max() <= 1e-5 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("sr", range(3))
+@pytest.mark.parametrize("name", list(CASES))
+def test_left_word_fold(name, sr):
+    """x^T M at one word per value: rows beyond one chunk of x, targets in
+    several blocks of 65,536 (rules, then terminals), and an x off the 16-byte
+    boundary, which takes the edge lists instead."""
+    import torch
+
+    m = CASES[name]()
+    rows, cols, codes, V = m.rows, m.cols, m.codes(), m.values()
+    r = np.repeat(np.arange(rows), np.diff(np.r_[-1, np.flatnonzero(codes == 0)]) - 1)
+    nz = codes[codes != 0].astype(np.int64) - 1
+    c, v = nz % cols, V[nz // cols]
+    plan = gmr.Plan.build(gmr.repair(m, device=0), rows, cols, device=0)
+    eng = gmr.Engine(plan)
+    eng.enable_left(plan)
+    rng = np.random.default_rng(8)
+    if sr == 0:
+        x = rng.uniform(-1, 1, rows).astype(np.float32)
+        ref = np.bincount(c, v * x[r].astype(np.float64), cols)
+    elif sr == 1:
+        x = np.where(rng.random(rows) < 3.0 / rows, rng.integers(1, 2**32, rows, dtype=np.uint64), 0).astype(np.uint32)
+        ref = np.zeros(cols, dtype=np.uint32)
+        np.bitwise_or.at(ref, c, x[r])
+    else:
+        x = np.where(rng.random(rows) < 0.01, rng.integers(0, 1000, rows), 2**31 - 1).astype(np.int32)
+        ref = np.full(cols, INF, dtype=np.int64)
+        np.minimum.at(ref, c, np.where(x[r] >= INF, INF, v.astype(np.int64) + x[r]))
+    buf = torch.zeros(rows + 4, dtype=torch.int32, device="cuda")
+    for offset in (0, 1):
+        buf[offset:offset + rows] = torch.from_numpy(x.view(np.int32)).cuda()
+        for _ in range(3):
+            dY = torch.full((cols,), 7, dtype=torch.int32, device="cuda")
+            eng.multiply_left_device(sr, buf.data_ptr() + 4 * offset, dY.data_ptr(), 32 if sr == 1 else 1)
+            torch.cuda.synchronize()
+        y = dY.cpu().numpy().view(x.dtype)
+        if sr == 0:
+            assert np.abs(y - ref).max() <= 1e-5 * np.abs(ref).max()
+        else:
+            np.testing.assert_array_equal(y, ref)
