@@ -1708,7 +1708,6 @@ static Launch resolve_launch(gmr_engine* e, int semiring, int B, const void* X, 
     if (lc.variant == GMR_VARIANT_PLAIN) lc.emit = GMR_EMIT_ATOMIC;
     lc.push_mode = cfg ? cfg->push : GMR_PUSH_AUTO;
     if (lc.push_mode < GMR_PUSH_AUTO || lc.push_mode > GMR_PUSH_INTERLEAVE) throw Error(GMR_ERR_ARG, "unknown push mode");
-    lc.chunk = cfg && cfg->ops_per_cta > 0 ? cfg->ops_per_cta : 16;
     auto aligned = [&](size_t al) { return ((uintptr_t)X % al == 0) && ((uintptr_t)Y % al == 0); };
     const bool tile_asked = cfg && cfg->vec_tile > 0 && cfg->vec_tile <= lc.Bw && lc.Bw % cfg->vec_tile == 0;
     int bt = tile_asked ? cfg->vec_tile : cfg && cfg->vec_tile > 0 ? lc.Bw : auto_tile(e, lc.Bw);  // tiles must divide the batch
@@ -1746,6 +1745,10 @@ static Launch resolve_launch(gmr_engine* e, int semiring, int B, const void* X, 
     else if (lc.Bt % 2 == 0 && lc.Bw % 2 == 0 && aligned(8)) lc.VEC = 2;
     else lc.VEC = 1;
     lc.G = lc.Bt / lc.VEC;
+    // measured over whole multiplies, 98,160 x 7,210: chunks of 32 against 16 take
+    // 805 and 827 us for (+,x) B = 32, 936 and 1005 for (min,+) B = 32, but 495 and
+    // 468 for (+,x) B = 8 (two lanes per value)
+    lc.chunk = cfg && cfg->ops_per_cta > 0 ? cfg->ops_per_cta : lc.G >= 4 ? 32 : 16;
     lc.word = e->word.ready && lc.Bw == 1 && max_vec >= 8 && lc.push_mode == GMR_PUSH_AUTO &&
               (lc.variant == GMR_VARIANT_GRAPH || lc.variant == GMR_VARIANT_FUSED) &&
               !(cfg && (cfg->emit_mode || cfg->ops_per_cta > 0)) &&
@@ -2048,9 +2051,10 @@ static void build_push_lists(const gmr_plan& p, gmr_engine& e) {
 // product's when left_terms >= 0 (its terminals' first target).  Not built where
 // it does not pay: graphs with direct terminals (their terminals are no table),
 // too few emissions, runs too short (kWordMinPerRow).
-static void build_word_list(gmr_engine& e, WordList& l, int64_t values, int64_t targets, int64_t left_terms) {
+static void build_word_list(gmr_engine& e, WordList& l, int64_t values, int64_t targets, int64_t left_terms,
+                            int64_t min_emissions) {
     const int64_t E = e.n_em, chunks = (values + kWordChunk - 1) / kWordChunk, blks = (targets + 65535) / 65536;
-    if (l.ready || e.direct_terms || e.n_ops == 0 || E < kWordMinEmissions || E >= (int64_t)UINT32_MAX - 1 ||
+    if (l.ready || e.direct_terms || e.n_ops == 0 || E < min_emissions || E >= (int64_t)UINT32_MAX - 1 ||
         (double)E < kWordMinPerRow * (double)chunks * (double)targets || chunks * blks > (1 << 20))
         return;
     const int row_bits = std::max(16, bits_for((uint64_t)targets));  // at least the 16 bits an entry keeps
@@ -2092,7 +2096,7 @@ static void build_word_list(gmr_engine& e, WordList& l, int64_t values, int64_t 
 
 static void build_word_fold(gmr_engine& e) {
     const int64_t values = word_t_span(e.n_terms) + e.n_ops, chunks = (values + kWordChunk - 1) / kWordChunk;
-    build_word_list(e, e.word, values, e.rows, -1);
+    build_word_list(e, e.word, values, e.rows, -1, kWordMinEmissions);
     e.word_copies = (int)std::min<int64_t>(kWordMaxCopies, (chunks + kWordChunksPerCopy - 1) / kWordChunksPerCopy);
     if (!e.word.ready || e.word_copies == 1) return;
     if (!build_order([&] { e.word_parts.ensure((size_t)e.rows * e.word_copies * 4); })) e.word_copies = 1;
@@ -2671,12 +2675,10 @@ __global__ void __launch_bounds__(256, VEC == 8 ? 4 : 5) k_left_fold(LeftArgs a)
 // that straddles two groups also straddles two chunks and starts at zero.
 static constexpr int kLeftGroup = 128;
 
-// Edges per lane group on a level of n edges: kLeftChunk, fewer on levels that
-// do not fill the GPU (the rounds of four edges are their time).
-static int left_chunk(int64_t n) {
-    static_assert(kLeftGroup % kLeftChunk == 0 && kLeftChunk == 16, "chunks divide a group");
-    return n <= (1 << 16) ? 4 : n <= (1 << 18) ? 8 : (int)kLeftChunk;
-}
+// Edges per lane group on a level of n edges (every choice divides kLeftGroup):
+// few on levels that do not fill the GPU, where the rounds of four edges are the
+// time (32 on the widest ones measured the same as 16).
+static int left_chunk(int64_t n) { return n <= (1 << 16) ? 4 : n <= (1 << 18) ? 8 : 16; }
 
 // ADD: every target already holds a value (the rows' part, from k_word_fold),
 // and sums are added to it.
@@ -2920,7 +2922,8 @@ extern "C" int gmr_engine_enable_left(gmr_engine* e, gmr_plan* p) {
             e->le_first = std::move(first);
         }
         // the rows' edges once more for the one-word fold, and the parents' alone
-        build_word_list(*e, e->left_word, e->rows, left_word_terms(e) + e->n_terms, left_word_terms(e));
+        build_word_list(*e, e->left_word, e->rows, left_word_terms(e) + e->n_terms, left_word_terms(e),
+                        kLeftWordMinEmissions);
         if (e->left_word.ready) {
             const int D = e->depth;
             std::vector<int32_t> src, tgt;
@@ -3988,9 +3991,10 @@ static void run_legacy(int rows, int cols, int alpha, int total_layered_rules, c
     cudaEventCreate(&t0);
     cudaEventCreate(&t1);
     gmr_config cfg{};
-    // warm-up: builds the graph outside the timed window
-    if (gmr_engine_multiply(eng, semiring, dX.p, dY.p, B, &cfg, nullptr) != GMR_OK)
-        legacy_fail("gmr_engine_multiply", gmr_last_error());
+    // warm-up: the second call captures the graph (run_chain), outside the timed window
+    for (int w = 0; w < 2; ++w)
+        if (gmr_engine_multiply(eng, semiring, dX.p, dY.p, B, &cfg, nullptr) != GMR_OK)
+            legacy_fail("gmr_engine_multiply", gmr_last_error());
     cudaEventRecord(t0, 0);
     for (int it = 0; it < iters; ++it)
         if (gmr_engine_multiply(eng, semiring, dX.p, dY.p, B, &cfg, nullptr) != GMR_OK)

@@ -41,6 +41,9 @@ constexpr int kWordGroup = 128;     // emissions per warp step: four per lane
 // 119 -> 64).
 constexpr double kWordMinPerRow = 0.25;
 constexpr int64_t kWordMinEmissions = 1 << 16, kWordMinEmissionsPlus = 2 << 20;
+// The left product pays two launches for it, about 10 us, and saves 26 us at
+// 15 M emissions (50,000 x 5,000); at 0.5 M (1,479 x 2,064) it lost 27 -> 37 us.
+constexpr int64_t kLeftWordMinEmissions = 6 << 20;
 // Chunks per copy of Y: a row gets one addition per chunk that emits into it,
 // and the error of that chain grows with its length.
 constexpr int kWordChunksPerCopy = 16, kWordMaxCopies = 16;

@@ -55,15 +55,19 @@ def test_word_fold(name, sr):
         assert np.abs(a - b).max() <= 1e-5 * np.abs(b).max()
 
 
+# the left product's list starts at 6 M emissions; "graph" stays on the edge lists
+LEFT = {"two_chunks_of_x": lambda: gmr.gen_mosaic(70001, 1500, 64, 0.01, 1e-3, 3), "graph": CASES["graph"]}
+
+
 @pytest.mark.parametrize("sr", range(3))
-@pytest.mark.parametrize("name", list(CASES))
+@pytest.mark.parametrize("name", list(LEFT))
 def test_left_word_fold(name, sr):
     """x^T M at one word per value: rows beyond one chunk of x, targets in
     several blocks of 65,536 (rules, then terminals), and an x off the 16-byte
     boundary, which takes the edge lists instead."""
     import torch
 
-    m = CASES[name]()
+    m = LEFT[name]()
     rows, cols, codes, V = m.rows, m.cols, m.codes(), m.values()
     r = np.repeat(np.arange(rows), np.diff(np.r_[-1, np.flatnonzero(codes == 0)]) - 1)
     nz = codes[codes != 0].astype(np.int64) - 1
@@ -95,3 +99,27 @@ def test_left_word_fold(name, sr):
             assert np.abs(y - ref).max() <= 1e-5 * np.abs(ref).max()
         else:
             np.testing.assert_array_equal(y, ref)
+
+
+def test_fixpoint_with_word_fold():
+    """The device loop runs the one-launch fold in its body: reachability of 32
+    sets against the per-level folds iterated from the host."""
+    import torch
+
+    m = CASES["graph"]()
+    n = m.rows
+    eng = gmr.Engine(gmr.Plan.build(gmr.repair(m, device=0), n, n, device=0))
+    x = np.zeros((n, 1), dtype=np.uint32)
+    x[np.arange(32) * 600, 0] = np.uint32(1) << np.arange(32, dtype=np.uint32)
+    dX = torch.from_numpy(x.view(np.int32)).cuda()
+    dY = torch.empty_like(dX)
+    iters = eng.fixpoint_device("boolean", dX.data_ptr(), dY.data_ptr(), 32)
+    ref, k = x, 0
+    while True:
+        nxt = ref | eng.multiply(ref, 1, B=32, push=gmr.PUSH_NEVER)
+        k += 1
+        if (nxt == ref).all():
+            break
+        ref = nxt
+    np.testing.assert_array_equal(dX.cpu().numpy().view(np.uint32), ref)
+    assert iters == k
