@@ -202,12 +202,21 @@ __global__ void __launch_bounds__(kWordThreads, 1) k_word_fold(WordFoldArgs a) {
             loaded = chunk;
         }
         constexpr int kWarps = kWordThreads / 32;
-        for (int64_t g = at + warp; g < to; g += 2 * kWarps) {  // two groups of loads in flight
-            const bool two = g + kWarps < to;
-            const uint4 q0 = __ldg(a.entries + g * 32 + lane);
-            const uint4 q1 = two ? __ldg(a.entries + (g + kWarps) * 32 + lane) : q0;
+        // the loads of the next two groups are in flight while two are folded (left
+        // product, 50,000 x 5,000: 184 us without, 157 with; no difference where the
+        // list streams from HBM at 200,000 x 10,000)
+        const uint4* mine = a.entries + lane;
+        int64_t g = at + warp;
+        uint4 q0 = g < to ? __ldg(mine + g * 32) : make_uint4(0, 0, 0, 0);
+        uint4 q1 = g + kWarps < to ? __ldg(mine + (g + kWarps) * 32) : q0;
+        for (; g < to; g += 2 * kWarps) {
+            const bool two = g + kWarps < to, three = g + 2 * kWarps < to, four = g + 3 * kWarps < to;
+            const uint4 p0 = three ? __ldg(mine + (g + 2 * kWarps) * 32) : q0;
+            const uint4 p1 = four ? __ldg(mine + (g + 3 * kWarps) * 32) : q0;
             fold_word_group<S>(q0, vals, Y, lane);
             if (two) fold_word_group<S>(q1, vals, Y, lane);
+            q0 = p0;
+            q1 = p1;
         }
         at = to;
     }
