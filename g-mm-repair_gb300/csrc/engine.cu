@@ -12,15 +12,17 @@
 //   * values of one multiply live in an arena [slot][Bw] (Bw = B words per
 //     slot, right-hand sides innermost), slots level-major and child-sorted by
 //     the plan builder; identity pass-throughs are references, not copies;
-//   * a thread group of G = Bw / VEC lanes handles one rule or emission and
-//     moves VEC consecutive words per lane with 8- or 16-byte accesses;
+//   * a thread group of G lanes handles one rule or emission and moves VEC
+//     consecutive words per lane with up to 32-byte accesses; rows of X and Y no
+//     such access reaches go through padded copies;
 //   * one launch per level k evaluates the rules of level k AND folds the
 //     emissions of level k-1 (complete since the previous launch), so a
-//     multiply is D + 2 launches instead of the reference's 2D + 4;
-//   * emissions are sorted by (row, source): a warp reduces each row segment
-//     in registers (shuffles for (+,x), __reduce_or/min_sync for the
-//     idempotent semirings) and issues one atomic per segment;
-//   * the launch chain can be captured once into a CUDA graph and replayed.
+//     multiply is D + 2 launches instead of the reference's 2D + 4, each placed
+//     while the one before drains (programmatic dependent launch);
+//   * emissions are sorted by (row, source): each run of a row is reduced in
+//     registers and issues one atomic; with one 4-byte word per value all levels'
+//     emissions are folded at the end out of shared memory (word_fold.cuh);
+//   * the launch chain is captured into a graph at its second use and replayed.
 #include <cuda_runtime.h>
 #include <dlfcn.h>
 

@@ -271,7 +271,7 @@ enum {
     GMR_VARIANT_AUTO = 0,
     GMR_VARIANT_PLAIN = 1,   /* per-level launches, one atomic per emission */
     GMR_VARIANT_FUSED = 2,   /* per-level launches, ops+emits fused */
-    GMR_VARIANT_GRAPH = 3,   /* FUSED captured once into a CUDA graph */
+    GMR_VARIANT_GRAPH = 3,   /* FUSED, captured into a CUDA graph at its second use */
     GMR_VARIANT_PERSISTENT = 4 /* one cooperative launch walks every level */
 };
 enum {
