@@ -512,6 +512,7 @@ __device__ __forceinline__ void do_emits_atomic(const SweepArgs& a, const LevelA
 template <class S, int VEC, bool CG = false, bool DIR = false>
 __device__ __forceinline__ void do_emits_warp(const SweepArgs& a, const LevelArgs& L, int tile, const Span& sp) {
     using T = typename S::T;
+    if (L.n_em == 0) return;
     const Values<S, VEC, CG> val(a, tile);
     const int lane = threadIdx.x & 31;
     const int64_t first = L.em_first, end = first + L.n_em, base = first & ~(int64_t)3;
@@ -559,6 +560,10 @@ __device__ __forceinline__ void do_emits_warp(const SweepArgs& a, const LevelArg
 template <class S, int VEC, int GLOG, bool CG = false, bool DIR = false>
 __device__ __forceinline__ void do_emits_chunk(const SweepArgs& a, const LevelArgs& L, int tile, const Span& sp) {
     using T = typename S::T;
+    // a level without emissions has no group: its first quad belongs to the levels
+    // beside it, or lies past the last emission (the per-level launches give such a
+    // level no blocks, the single-kernel sweeps walk every level)
+    if (L.n_em == 0) return;
     const Values<S, VEC, CG> val(a, tile);
     const int skew = (int)(L.em_first & 3);  // emissions of the first quad that belong to the level below
     const int64_t base = L.em_first - skew, n = L.n_em + skew;
