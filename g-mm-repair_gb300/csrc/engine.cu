@@ -201,7 +201,10 @@ __device__ __forceinline__ void vred(typename S::T* p, const Vec<typename S::T, 
 // the current one drains, and wait here before they touch anything it wrote.
 // griddepcontrol.wait returns when the kernel before has completed and its
 // writes are visible; every block of every chained kernel executes it, so a
-// kernel that has completed implies all before it have.  What a launch
+// kernel that has completed implies all before it have.  What an earlier kernel
+// of the chain writes is read by plain loads through plain pointers: a const
+// __restrict__ parameter or __ldg would promise that it does not change while
+// this kernel runs, waiting included.  What a launch
 // boundary costs is what bounds the narrow levels (2.0 us each, of which the
 // rules and emissions of such a level need well under 1 us).  Measured, one
 // multiply as a graph: 36.6 -> 29.4 us for 2,000 x 1,000 at B = 1 (19
@@ -419,10 +422,11 @@ __global__ void __launch_bounds__(256) k_prologue(SweepArgs a) {
 
 // Rows of `from` words (stride ldi) copied to rows of ldo words: the padded
 // copy of X (the words past `from` are the semiring zero) and the caller's Y
-// from its padded copy (ldo = from: nothing to pad).
+// from its padded copy (ldo = from: nothing to pad).  `in` may be written by the
+// kernel before, which this one overlaps until the wait: no __restrict__, which
+// would let its loads go ahead of the wait or down the read-only path.
 template <class T>
-__global__ void __launch_bounds__(256) k_restride(const T* __restrict__ in, T* __restrict__ out, int64_t rows, int from,
-                                                  int ldi, int ldo, T pad) {
+__global__ void __launch_bounds__(256) k_restride(const T* in, T* out, int64_t rows, int from, int ldi, int ldo, T pad) {
     dependents_may_launch();
     wait_for_previous_kernel();
     const Span sp = span_of<-1>(ldo, blockIdx.x, gridDim.x);

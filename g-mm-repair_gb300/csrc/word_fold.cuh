@@ -222,15 +222,14 @@ __global__ void __launch_bounds__(kWordThreads, 1) k_word_fold(WordFoldArgs a) {
     }
 }
 
-// Y from its copies.
+// Y from its copies, which the fold before writes (plain loads, no __restrict__).
 template <class S>
-__global__ void __launch_bounds__(256) k_word_sum(const typename S::T* __restrict__ parts, typename S::T* __restrict__ Y,
-                                                  int64_t rows, int copies) {
+__global__ void __launch_bounds__(256) k_word_sum(const typename S::T* parts, typename S::T* Y, int64_t rows, int copies) {
     dependents_may_launch();
     wait_for_previous_kernel();
     for (int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x; r < rows; r += (int64_t)gridDim.x * 256) {
-        typename S::T v = __ldcg(parts + r);
-        for (int c = 1; c < copies; ++c) v = S::oplus(v, __ldcg(parts + c * rows + r));
+        typename S::T v = parts[r];
+        for (int c = 1; c < copies; ++c) v = S::oplus(v, parts[c * rows + r]);
         Y[r] = v;
     }
 }
