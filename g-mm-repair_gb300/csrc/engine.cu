@@ -516,7 +516,6 @@ __device__ __forceinline__ void do_emits_atomic(const SweepArgs& a, const LevelA
 template <class S, int VEC, bool CG = false, bool DIR = false>
 __device__ __forceinline__ void do_emits_warp(const SweepArgs& a, const LevelArgs& L, int tile, const Span& sp) {
     using T = typename S::T;
-    if (L.n_em == 0) return;
     const Values<S, VEC, CG> val(a, tile);
     const int lane = threadIdx.x & 31;
     const int64_t first = L.em_first, end = first + L.n_em, base = first & ~(int64_t)3;
@@ -561,13 +560,11 @@ __device__ __forceinline__ void do_emits_warp(const SweepArgs& a, const LevelArg
 // indices, because the groups' chunks lie 64 bytes apart.  Indices are
 // therefore read four at a time (one 16-byte load instead of four 4-byte
 // ones): with single loads they took as many tag cycles as the values.
+// Callers: L.n_em > 0 (the first quad of a level without emissions belongs to the
+// levels beside it, or lies past the last emission).
 template <class S, int VEC, int GLOG, bool CG = false, bool DIR = false>
 __device__ __forceinline__ void do_emits_chunk(const SweepArgs& a, const LevelArgs& L, int tile, const Span& sp) {
     using T = typename S::T;
-    // a level without emissions has no group: its first quad belongs to the levels
-    // beside it, or lies past the last emission (the per-level launches give such a
-    // level no blocks, the single-kernel sweeps walk every level)
-    if (L.n_em == 0) return;
     const Values<S, VEC, CG> val(a, tile);
     const int skew = (int)(L.em_first & 3);  // emissions of the first quad that belong to the level below
     const int64_t base = L.em_first - skew, n = L.n_em + skew;
@@ -855,7 +852,7 @@ __global__ void __launch_bounds__(256) k_persistent(SweepArgs a, LevelArgs L0, P
         L.n_em = P.em_off[k] - P.em_off[k - 1];
         L.seg_first = P.seg_off[k - 1];
         L.n_seg = P.seg_off[k] - P.seg_off[k - 1];
-        emits_t<S, VEC, GLOG, EMIT, true, false>(a, L, 0, sp);
+        if (L.n_em > 0) emits_t<S, VEC, GLOG, EMIT, true, false>(a, L, 0, sp);
         do_ops<S, VEC, GLOG, true, false>(a, L, 0, sp);
         if (!grid_barrier(P, k)) return;
     }
@@ -899,7 +896,7 @@ __device__ __forceinline__ void pack_phase(const PackGrammar& g, int k) {
     L.n_em = g.em_off[k] - g.em_off[k - 1];
     L.seg_first = g.seg_off[k - 1];
     L.n_seg = g.seg_off[k] - g.seg_off[k - 1];
-    emits_t<S, VEC, GLOG, EMIT, true, false>(a, L, 0, sp);
+    if (L.n_em > 0) emits_t<S, VEC, GLOG, EMIT, true, false>(a, L, 0, sp);
     do_ops<S, VEC, GLOG, true, false>(a, L, 0, sp);
 }
 
