@@ -1779,10 +1779,19 @@ static void drop_oldest_graph(gmr_engine* e) {
 // time, replayed from then on (the engine remembers 8 sets of arguments).
 // Capturing and instantiating costs more than a small multiply (0.4 ms for 24
 // launches, against 0.1 ms for launching them), which a caller with new
-// buffers on every call would pay each time.
+// buffers on every call would pay each time.  On a stream that the caller is
+// capturing the launches go into the caller's graph: a capture or an
+// instantiation of the engine's own would break the caller's.
 template <class F>
 static int64_t run_chain(gmr_engine* e, const Launch& lc, GraphEntry::Kind kind, const void* X, void* Y,
                          cudaStream_t st, F&& chain) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) cudaGetLastError();  // not this stream's: the launches say
+    if (capturing != cudaStreamCaptureStatusNone) {
+        int64_t n = 0;
+        chain(st, n);
+        return n;
+    }
     GraphEntry* hit = nullptr;
     for (auto& g : e->graphs)
         if (g.kind == kind && g.lc == lc && g.X == X && g.Y == Y) hit = &g;
@@ -1811,9 +1820,11 @@ static int64_t run_chain(gmr_engine* e, const Launch& lc, GraphEntry::Kind kind,
             throw;
         }
         GMR_CUDA(cudaStreamEndCapture(e->own_stream, &graph));
-        cudaError_t ie = cudaGraphInstantiate(&hit->exec, graph, 0);
+        cudaGraphExec_t exec = nullptr;
+        cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
         cudaGraphDestroy(graph);
         GMR_CUDA(ie);
+        hit->exec = exec;
         hit->launches = n;
     }
     GMR_CUDA(cudaGraphLaunch(hit->exec, st));
