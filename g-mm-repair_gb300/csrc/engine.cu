@@ -38,6 +38,7 @@
 #include <mutex>
 #include <string>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "gmr_internal.h"
@@ -2068,15 +2069,17 @@ static void build_push_lists(const gmr_plan& p, gmr_engine& e) {
     }
 }
 
-// A (chunk, target) order of the emissions for k_word_fold, sorted on the GPU
-// from the uploaded ones: of `values` values into `targets` targets, the left
-// product's when left_terms >= 0 (its terminals' first target).  Not built where
+// A (chunk, target) order of the E emissions src, row for k_word_fold, sorted on
+// the GPU: of `values` values into `targets` targets, the left product's when
+// left_terms >= 0 (its terminals' first target).  emissions() gives the device
+// arrays; it is called once it is known that the list pays.  Not built where
 // it does not pay: graphs with direct terminals (their terminals are no table),
 // too few emissions, runs too short (kWordMinPerRow).
-static void build_word_list(gmr_engine& e, WordList& l, int64_t values, int64_t targets, int64_t left_terms,
-                            int64_t min_emissions) {
-    const int64_t E = e.n_em, chunks = (values + kWordChunk - 1) / kWordChunk, blks = (targets + 65535) / 65536;
-    if (l.ready || e.direct_terms || e.n_ops == 0 || E < min_emissions || E >= (int64_t)UINT32_MAX - 1 ||
+template <class F>
+static void build_word_list(gmr_engine& e, WordList& l, F&& emissions, int64_t E, int64_t values, int64_t targets,
+                            int64_t left_terms, int64_t min_emissions) {
+    const int64_t chunks = (values + kWordChunk - 1) / kWordChunk, blks = (targets + 65535) / 65536;
+    if (e.direct_terms || e.n_ops == 0 || E < min_emissions || E >= (int64_t)UINT32_MAX - 1 ||
         (double)E < kWordMinPerRow * (double)chunks * (double)targets || chunks * blks > (1 << 20))
         return;
     const int row_bits = std::max(16, bits_for((uint64_t)targets));  // at least the 16 bits an entry keeps
@@ -2085,9 +2088,9 @@ static void build_word_list(gmr_engine& e, WordList& l, int64_t values, int64_t 
     const bool built = build_order([&] {
         DevArray<uint64_t> ka(E), kb(E);
         DevArray<uint32_t> tmp(dev::sort_scratch(E) + 1), first(n_seg + 1);
-        k_word_keys<<<dev::grid_for(E), 256>>>(static_cast<const int32_t*>(e.em_src.p),
-                                               static_cast<const int32_t*>(e.em_row.p), E, word_t_span(e.n_terms),
-                                               row_bits, left_terms >= 0, left_terms, ka.p);
+        const std::pair<const int32_t*, const int32_t*> em = emissions();
+        k_word_keys<<<dev::grid_for(E), 256>>>(em.first, em.second, E, word_t_span(e.n_terms), row_bits, left_terms >= 0,
+                                               left_terms, ka.p);
         uint64_t *k1 = ka.p, *k2 = kb.p;
         uint32_t *v1 = nullptr, *v2 = nullptr;
         dev::radix_sort(k1, k2, v1, v2, E, row_bits + bits_for((uint64_t)chunks), tmp.p, nullptr);
@@ -2118,7 +2121,10 @@ static void build_word_list(gmr_engine& e, WordList& l, int64_t values, int64_t 
 
 static void build_word_fold(gmr_engine& e) {
     const int64_t values = word_t_span(e.n_terms) + e.n_ops, chunks = (values + kWordChunk - 1) / kWordChunk;
-    build_word_list(e, e.word, values, e.rows, -1, kWordMinEmissions);
+    auto emissions = [&] {
+        return std::pair(static_cast<const int32_t*>(e.em_src.p), static_cast<const int32_t*>(e.em_row.p));
+    };
+    build_word_list(e, e.word, emissions, e.n_em, values, e.rows, -1, kWordMinEmissions);
     e.word_copies = (int)std::min<int64_t>(kWordMaxCopies, (chunks + kWordChunksPerCopy - 1) / kWordChunksPerCopy);
     if (!e.word.ready || e.word_copies == 1) return;
     if (!build_order([&] { e.word_parts.ensure((size_t)e.rows * e.word_copies * 4); })) e.word_copies = 1;
@@ -2922,10 +2928,22 @@ extern "C" int gmr_engine_enable_left(gmr_engine* e, gmr_plan* p) {
         if (!e || !p) throw Error(GMR_ERR_ARG, "null argument");
         if (p->n_ops() != e->n_ops || p->rows != e->rows || p->cols != e->cols)
             throw Error(GMR_ERR_ARG, "plan does not match the engine");
+        if (p->depth != e->depth || p->n_terms() > e->n_terms)  // its levels and terminals index the engine's
+            throw Error(GMR_ERR_ARG, "plan does not match the engine");
         int rc = gmr_plan_prepare_left(p);
         if (rc != GMR_OK) throw Error(rc, gmr_last_error());
         std::lock_guard<std::mutex> lk(e->mu);
         DeviceGuard dg(e->device);
+        if (e->left_ready) {  // a new plan's lists: nothing of the old ones' stays, graphs and running products included
+            GMR_CUDA(cudaDeviceSynchronize());
+            e->left_ready = false;
+            e->left_word.ready = false;
+            auto& gs = e->graphs;
+            for (auto& g : gs)
+                if (g.kind == GraphEntry::kLeft && g.exec) cudaGraphExecDestroy(g.exec);
+            gs.erase(std::remove_if(gs.begin(), gs.end(), [](const GraphEntry& g) { return g.kind == GraphEntry::kLeft; }),
+                     gs.end());
+        }
         {
             // each level's list from a multiple of four on: edges are read in aligned quads
             const int D = e->depth;
@@ -2943,9 +2961,23 @@ extern "C" int gmr_engine_enable_left(gmr_engine* e, gmr_plan* p) {
             }
             e->le_first = std::move(first);
         }
-        // the rows' edges once more for the one-word fold, and the parents' alone
-        build_word_list(*e, e->left_word, e->rows, left_word_terms(e) + e->n_terms, left_word_terms(e),
-                        kLeftWordMinEmissions);
+        // the rows' edges once more for the one-word fold (from this plan's emissions,
+        // which need not be the engine's own), and the parents' alone
+        {
+            DevBuf src, row;
+            struct Release {
+                DevBuf &a, &b;
+                ~Release() {
+                    a.release();
+                    b.release();
+                }
+            } release{src, row};
+            auto emissions = [&] {
+                return std::pair<const int32_t*, const int32_t*>(upload(p->em_src, src), upload(p->em_row, row));
+            };
+            build_word_list(*e, e->left_word, emissions, (int64_t)p->em_src.size(), e->rows,
+                            left_word_terms(e) + e->n_terms, left_word_terms(e), kLeftWordMinEmissions);
+        }
         if (e->left_word.ready) {
             const int D = e->depth;
             std::vector<int32_t> src, tgt;
