@@ -12,11 +12,15 @@
 
 namespace gmr {
 
+// The error is taken off the runtime's record: a later call's look at
+// cudaGetLastError would otherwise report it as its own.
 #define GMR_CUDA(call)                                                                                  \
     do {                                                                                                \
         cudaError_t err_ = (call);                                                                      \
-        if (err_ != cudaSuccess)                                                                        \
+        if (err_ != cudaSuccess) {                                                                      \
+            cudaGetLastError();                                                                         \
             throw ::gmr::Error(GMR_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(err_));    \
+        }                                                                                               \
     } while (0)
 
 struct DevBuf {

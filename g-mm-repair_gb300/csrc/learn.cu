@@ -32,8 +32,10 @@ namespace gmr {
 #define GMR_LCUDA(call)                                                                                \
     do {                                                                                               \
         cudaError_t err_ = (call);                                                                     \
-        if (err_ != cudaSuccess)                                                                       \
+        if (err_ != cudaSuccess) {                                                                     \
+            cudaGetLastError(); /* not a later call's */                                               \
             throw ::gmr::Error(GMR_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(err_));   \
+        }                                                                                              \
     } while (0)
 
 // ------------------------------------------------------------------ kernels
