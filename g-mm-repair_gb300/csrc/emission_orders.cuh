@@ -66,12 +66,20 @@ static __global__ void __launch_bounds__(256) k_chunk_keys(const int32_t* __rest
 }
 
 // first[g] for g = 0..groups: the first j whose key's low 32 bits are g or more.
+// A search per group: its time does not depend on how the keys lie (one thread
+// per key that fills the groups since the key before it walks whole levels that
+// emit nothing alone).
 template <class T>
 __global__ void __launch_bounds__(256) k_group_firsts(const uint64_t* __restrict__ key, int64_t n, int64_t groups,
                                                       T* __restrict__ first) {
-    for (int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x; j <= n; j += (int64_t)gridDim.x * 256) {
-        const int64_t prev = j ? (int64_t)(uint32_t)key[j - 1] : -1, cur = j < n ? (int64_t)(uint32_t)key[j] : groups;
-        for (int64_t g = prev + 1; g <= cur && g <= groups; ++g) first[g] = (T)j;
+    for (int64_t g = (int64_t)blockIdx.x * 256 + threadIdx.x; g <= groups; g += (int64_t)gridDim.x * 256) {
+        int64_t lo = 0, hi = n;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if ((int64_t)(uint32_t)key[mid] < g) lo = mid + 1;
+            else hi = mid;
+        }
+        first[g] = (T)lo;
     }
 }
 

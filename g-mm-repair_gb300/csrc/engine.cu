@@ -1955,7 +1955,7 @@ static void build_chunked_emissions(const gmr_plan& p, gmr_engine& e) {
         uint64_t *k1 = ka.p, *k2 = kb.p;
         uint32_t *v1 = va.p, *v2 = vb.p;
         dev::radix_sort(k1, k2, v1, v2, E, bits_for((uint64_t)groups), tmp.p, nullptr);
-        orders::k_group_firsts<<<dev::grid_for(E + 1), 256>>>(k1, E, groups, first.p);
+        orders::k_group_firsts<<<dev::grid_for(groups + 1), 256>>>(k1, E, groups, first.p);
         e.em_src_c.ensure((size_t)E * 4 + 16);
         e.em_row_c.ensure((size_t)E * 4 + 16);
         GMR_CUDA(cudaMemcpyAsync(e.em_src_c.p, v1, (size_t)E * 4, cudaMemcpyDeviceToDevice, nullptr));
@@ -2057,7 +2057,7 @@ static void build_push_lists(const gmr_plan& p, gmr_engine& e) {
             dev::radix_sort(k1, k2, v1, v2, n, bits_for((uint64_t)n_ops), tmp.p, nullptr);
             GMR_CUDA(cudaMemcpyAsync(e.pe_row.p, v1, (size_t)n * 4, cudaMemcpyDeviceToDevice, nullptr));
         }
-        orders::k_group_firsts<<<dev::grid_for(n + 1), 256>>>(k1, n, n_ops, static_cast<int32_t*>(e.pe_off.p));
+        orders::k_group_firsts<<<dev::grid_for(n_ops + 1), 256>>>(k1, n, n_ops, static_cast<int32_t*>(e.pe_off.p));
         GMR_CUDA(cudaGetLastError());
         std::vector<uint8_t> m((size_t)D + 2);
         GMR_CUDA(cudaMemcpy(m.data(), mixed.p, m.size(), cudaMemcpyDeviceToHost));
