@@ -118,6 +118,7 @@ void validate_plan(const gmr_plan& p);  // throws Error(GMR_ERR_FORMAT)
 void fill_common_stats(gmr_plan& p);    // stats derived from the plan arrays
 }
 
+#include <system_error>
 #include <thread>
 namespace gmr {
 template <class F>
@@ -128,7 +129,17 @@ void parallel_for_threads(int n_threads, F&& f) {
     }
     std::vector<std::thread> th;
     th.reserve(n_threads);
-    for (int t = 0; t < n_threads; ++t) th.emplace_back([&f, t] { f(t); });
-    for (auto& x : th) x.join();
+    struct Join {
+        std::vector<std::thread>& th;
+        ~Join() {
+            for (auto& x : th) x.join();
+        }
+    } join{th};
+    int t = 0;
+    try {
+        for (; t < n_threads; ++t) th.emplace_back([&f, t] { f(t); });
+    } catch (const std::system_error&) {  // no more threads to be had: this one does the rest
+    }
+    for (; t < n_threads; ++t) f(t);
 }
 }  // namespace gmr
