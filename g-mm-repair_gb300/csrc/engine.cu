@@ -1338,11 +1338,6 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
             if (v % kNumEmitVariants == 0) chunk = lc.G >= 4 ? 32 : 16;
             ops_cap = kOpsCtasPerSm[(v / kNumEmitVariants) % 2];
             by_chunk = v >= 2 * kNumEmitVariants;
-            // with one lane per value the warp fold beats the row-owned and the
-            // atomic one on every level (98,160 x 7,210, 128 Boolean columns: 416
-            // us a multiply against 553 and 1870; (+,x) B = 4: 402, 555, 706), and
-            // tables made before it was the fastest still ask for those
-            if (GLOG == 0) emit = GMR_EMIT_SEGMENTED;
         }
         if (lc.variant == GMR_VARIANT_PLAIN) emit = GMR_EMIT_ATOMIC;
         // level k_em pushed its emissions in its own launch: nothing to fold
@@ -1761,12 +1756,23 @@ static Launch resolve_launch(gmr_engine* e, int semiring, int B, const void* X, 
     // 805 and 827 us for (+,x) B = 32, 936 and 1005 for (min,+) B = 32, but 495 and
     // 468 for (+,x) B = 8 (two lanes per value)
     lc.chunk = cfg && cfg->ops_per_cta > 0 ? cfg->ops_per_cta : lc.G >= 4 ? 32 : 16;
-    lc.word = e->word.ready && lc.Bw == 1 && max_vec >= 8 && lc.push_mode == GMR_PUSH_AUTO &&
+    // a table that asks for anything but the plain choice is for the per-level folds
+    const bool plain = lc.lv.empty() || std::all_of(lc.lv.begin() + 1, lc.lv.end(), [](uint8_t v) { return v == 0; });
+    lc.word = e->word.ready && lc.Bw == 1 && plain && max_vec >= 8 && lc.push_mode == GMR_PUSH_AUTO &&
               (lc.variant == GMR_VARIANT_GRAPH || lc.variant == GMR_VARIANT_FUSED) &&
               !(cfg && (cfg->emit_mode || cfg->ops_per_cta > 0)) &&
               (semiring != GMR_PLUS_TIMES || e->n_em >= kWordMinEmissionsPlus);
-    if (lc.word) lc.lv.clear();  // the tables choose among the per-level folds
+    if (lc.word) lc.lv.clear();
     return lc;
+}
+
+int table_lanes(gmr_engine* e, int semiring, int B) {
+    std::lock_guard<std::mutex> lk(e->mu);
+    gmr_config cfg{};
+    cfg.variant = GMR_VARIANT_GRAPH;  // no table: what the engine does without one
+    // 256-byte aligned stand-ins: only the alignment of X and Y enters the choice
+    const Launch lc = resolve_launch(e, semiring, B, reinterpret_cast<const void*>(256), reinterpret_cast<void*>(256), &cfg);
+    return lc.word ? 0 : lc.G;
 }
 
 static void drop_oldest_graph(gmr_engine* e) {
@@ -2360,7 +2366,14 @@ extern "C" int gmr_engine_autotune_energy(gmr_engine* e, int semiring, const voi
         std::vector<float> med((size_t)nl * nv, 0.f);
         std::vector<uint8_t> uni(nl);
         std::vector<float> buf((size_t)nl + 8);
+        // Where one launch folds every emission there is nothing to choose: the plain
+        // table keeps that fold, and its times stand for every variant.
+        const bool one_fold = table_lanes(e, semiring, B) == 0;
         for (int v = 0; v < nv; ++v) {
+            if (one_fold && v) {
+                for (int l = 0; l < nl; ++l) med[(size_t)l * nv + v] = med[(size_t)l * nv];
+                continue;
+            }
             std::fill(uni.begin(), uni.end(), (uint8_t)v);
             if (gmr_engine_set_level_variants(e, semiring, B, uni.data(), nl) != GMR_OK) throw Error(GMR_ERR_ARG, gmr_last_error());
             std::vector<std::vector<float>> runs;
@@ -2380,6 +2393,12 @@ extern "C" int gmr_engine_autotune_energy(gmr_engine* e, int semiring, const voi
             }
         }
         std::vector<uint8_t> best(nl, 0);
+        if (one_fold) {  // `uni` of zeros is installed
+            std::lock_guard<std::mutex> lk(e->mu);
+            e->mode_costs.erase({semiring, B});
+            if (ms) std::copy(med.begin(), med.end(), ms);
+            return;
+        }
         for (int l = 0; l < nl; ++l) {
             int b = 0;
             for (int v = 1; v < nv; ++v)

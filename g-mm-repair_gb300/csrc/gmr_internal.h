@@ -116,6 +116,9 @@ namespace gmr {
 constexpr int64_t kLeftChunk = 16;  // edges per lane group in the left fold
 void validate_plan(const gmr_plan& p);  // throws Error(GMR_ERR_FORMAT)
 void fill_common_stats(gmr_plan& p);    // stats derived from the plan arrays
+// Lanes per value of a multiply of (semiring, B), 0 where the engine folds all
+// emissions in one launch: what a per-launch table chooses among depends on it.
+int table_lanes(gmr_engine* e, int semiring, int B);
 }
 
 #include <system_error>

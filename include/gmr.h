@@ -316,8 +316,10 @@ int gmr_engine_time_launches(gmr_engine* e, int semiring, const void* dX, void* 
  * table is used by GMR_VARIANT_AUTO multiplies of that (semiring, B).
  * With one 4-byte word per value (B = 1, or up to 32 Boolean right-hand sides)
  * and enough emissions the engine folds every level's emissions in one launch
- * after the rules, and a table has nothing to choose; with one lane per value
- * (1, 2 or 4 words) e = 3 and 4 run the segmented fold, which is faster there.
+ * after the rules, unless a table with an entry other than 0 is installed: such
+ * a table's per-level folds run as it says.  Row-owned folds on every level
+ * (e = 3, or GMR_EMIT_ROWS) add each row's emissions in a fixed order; the
+ * segmented and atomic folds and the one-launch fold add in any order.
  * Adding GMR_LEVEL_PUSH to slot k's entry (1 <= k <= depth) makes the rules of
  * level k push their values into the rows that emit them as soon as they are
  * computed (vector reductions into Y, which stays in L2), so launch k+1
@@ -348,7 +350,9 @@ int gmr_engine_set_level_variants(gmr_engine* e, int semiring, int B, const uint
 int gmr_engine_get_level_variants(const gmr_engine* e, int semiring, int B, uint8_t* v, int cap, int* n);
 /* Exhaustive autotuner: times every variant on every launch (median of
  * `reps` eager runs with the timing recorder), installs the per-launch
- * fastest, and writes the times to ms[slot * GMR_N_LEVEL_VARIANTS + v]. */
+ * fastest, and writes the times to ms[slot * GMR_N_LEVEL_VARIANTS + v].  Where
+ * the engine folds all emissions in one launch (see above) it installs the plain
+ * table, writes that table's times for every variant and has no mode costs. */
 int gmr_engine_autotune(gmr_engine* e, int semiring, const void* dX, void* dY, int B,
                         void* stream, int reps, float* ms, int cap);
 /* The same, trading a little time for fewer DRAM bytes: a launch whose
@@ -400,7 +404,9 @@ int gmr_mlp_load(const char* path, gmr_mlp** out);
 void gmr_mlp_free(gmr_mlp* m);
 /* Predicts every variant's time on every launch of (semiring, B), installs
  * the per-launch argmin as the engine's table, writes the predictions (log us)
- * to pred[slot * GMR_N_LEVEL_VARIANTS + v] when pred != NULL. */
+ * to pred[slot * GMR_N_LEVEL_VARIANTS + v] when pred != NULL.  Variants that the
+ * engine's newer folds beat wherever they apply are not chosen: their prediction
+ * is +infinity. */
 int gmr_engine_choose_learned(gmr_engine* e, const gmr_plan* p, const gmr_mlp* m, int semiring, int B,
                               float* pred, int cap);
 
