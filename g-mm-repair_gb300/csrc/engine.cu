@@ -1333,9 +1333,6 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
             const int v = (lc.lv[slot] & ~(GMR_LEVEL_PUSH | GMR_LEVEL_INTERLEAVE | GMR_LEVEL_STAGE)) % GMR_N_LEVEL_VARIANTS;
             emit = kEmitVariants[v % kNumEmitVariants].emit;
             chunk = kEmitVariants[v % kNumEmitVariants].chunk;
-            // the plain choice, as without a table (200,000 x 10,000, B = 32, learned
-            // table: 1776 us a multiply with chunks of 16, 1720 with 32)
-            if (v % kNumEmitVariants == 0) chunk = lc.G >= 4 ? 32 : 16;
             ops_cap = kOpsCtasPerSm[(v / kNumEmitVariants) % 2];
             by_chunk = v >= 2 * kNumEmitVariants;
         }

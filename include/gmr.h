@@ -245,7 +245,9 @@ typedef struct {
     int variant;      /* GMR_VARIANT_* */
     int vec_tile;     /* words per right-hand-side tile (must divide the
                          batch's words; 0 = engine default) */
-    int ops_per_cta;  /* emissions per lane group in GMR_EMIT_SEGMENTED */
+    int ops_per_cta;  /* most emissions per lane group in GMR_EMIT_SEGMENTED:
+                         rounded up to a multiple of 4, halved on levels that
+                         do not fill the GPU, unused at one lane per value */
     int emit_mode;    /* GMR_EMIT_* */
     int tile_levels;  /* levels 1..tile_levels run tile by tile, the rest
                          all tiles per launch (0 = by level size) */
@@ -255,11 +257,13 @@ typedef struct {
                          the rows that emit them (see GMR_LEVEL_PUSH) */
     int lane_bytes;   /* bytes each lane moves per value access: 16, or 32
                          (256-bit loads and stores, 8 words per lane; used for
-                         (+,x) and (min,+) when the tile is 8, 16, 32, 64 or
-                         128 words and X and Y are 32-byte aligned, else 16);
-                         0 = engine default: 32 for (+,x) tiles of 32 words
-                         or more, else 16 (GMR_LANE_BYTES=16|32 at engine
-                         creation overrides it) */
+                         tiles of up to 128 words, multiples of 8 for (+,x)
+                         and 8, 16, 32, 64 or 128 for (min,+) and in
+                         GMR_VARIANT_PERSISTENT, when X and Y are 32-byte
+                         aligned or the batch is padded inside the engine,
+                         else 16); 0 = engine default: 32 for (+,x) tiles of
+                         32 words or more, else 16 (GMR_LANE_BYTES=16|32 at
+                         engine creation overrides it) */
 } gmr_config;
 enum {
     GMR_PUSH_AUTO = 0,       /* the installed per-launch table, else the engine's rule */
@@ -306,10 +310,11 @@ int gmr_engine_time_launches(gmr_engine* e, int semiring, const void* dX, void* 
 /* Per-launch kernel variants (the autotuner's and the learned model's
  * decision table).  Launch slot 0 is the prologue (ignored), slot k the launch
  * of level k (rules of level k + emissions of level k-1), slot depth+1 the
- * final fold.  Variant v = e + 5 * g + 10 * c: e = 0 segmented, chunk 16
- * (32 where four or more lanes hold a value), 1 chunk 8, 2 chunk 32 (for one lane
- * per emission all three are the warp fold; levels that do not fill the GPU halve
- * their chunk), 3 row-owned, 4 one atomic per emission; g = 0 up
+ * final fold.  Variant v = e + 5 * g + 10 * c: e = 0 segmented, chunk 16,
+ * 1 chunk 8, 2 chunk 32 (for one lane per emission all three are the warp fold;
+ * levels that do not fill the GPU halve their chunk; without a table the engine
+ * takes 32 where four or more lanes hold a value, else 16), 3 row-owned, 4 one
+ * atomic per emission; g = 0 up
  * to 32 CTAs per SM evaluate the rules, g = 1 up to 4 (more rules per CTA);
  * c = 1 folds the emissions one source chunk (2^19 slots of the level) at a
  * time, one launch per chunk, so the chunk's values stay in L2.  An installed

@@ -36,7 +36,8 @@ def test_row_owned_tables_add_in_a_fixed_order(mosaic, B):
 @pytest.mark.parametrize("sr,B", [(0, 1), (0, 2), (0, 4), (1, 32), (1, 128), (2, 1), (0, 32)])
 def test_learned_tables(mosaic, sr, B):
     """The installed table is the argmin of the returned predictions; plain where
-    one launch folds everything, no row-owned or atomic folds at one lane."""
+    one launch folds everything, no row-owned or atomic folds at one lane, no
+    chunks of 16 at four."""
     eng = gmr.Engine(mosaic)
     pred = learn.choose_learned(eng, mosaic, learn.Mlp.load(learn.MODEL_PATH), sr, B)
     table = eng.level_variants(sr, B)
@@ -46,6 +47,8 @@ def test_learned_tables(mosaic, sr, B):
         assert not table.any()
     elif words <= 4:
         assert not (table % 5).any()
+    else:  # four lanes: chunks of 32 in the place of 16
+        assert (table[1:] % 5).all()
 
 
 def test_autotuner_where_one_launch_folds_everything(mosaic):
