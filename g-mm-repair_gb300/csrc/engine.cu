@@ -1043,6 +1043,7 @@ struct gmr_engine {
     gmr::DevBuf ops, op_c, em_src, em_row, seg_row, seg_start, term_val, term_col, V;
     gmr::DevBuf arena, T, hX, hY;  // scratch
     gmr::DevBuf padX, padY;        // scratch: X and Y in padded rows (Launch::padded)
+    size_t pad_refused = SIZE_MAX;  // bytes of padded scratch the device did not have
     gmr::DevBuf hX2, hY2;          // second staging pair of the pipelined host-buffer multiply
     cudaStream_t copy_in = nullptr, copy_out = nullptr;
     cudaEvent_t pipe_ev[6] = {};    // per staging slot: X copied in, multiply done, Y copied out
@@ -1693,7 +1694,7 @@ static bool needs_padding(const gmr_engine* e, int semiring, int Bw, bool aligne
 static int padded_words(int Bw) { return Bw <= 4 ? 4 : (Bw + 7) / 8 * 8; }
 
 static Launch resolve_launch(gmr_engine* e, int semiring, int B, const void* X, void* Y, const gmr_config* cfg,
-                             int max_vec = 8) {
+                             int max_vec = 8, bool may_pad = true) {
     Launch lc{};
     lc.semiring = semiring;
     lc.B = B;
@@ -1717,7 +1718,7 @@ static Launch resolve_launch(gmr_engine* e, int semiring, int B, const void* X, 
     int bt = tile_asked ? cfg->vec_tile : cfg && cfg->vec_tile > 0 ? lc.Bw : auto_tile(e, lc.Bw);  // tiles must divide the batch
     if (lc.variant == GMR_VARIANT_PERSISTENT) bt = lc.Bw;  // one tile: the whole batch in one launch
     lc.Bp = lc.Bw;
-    lc.padded = max_vec >= 8 && lc.variant != GMR_VARIANT_PERSISTENT && !tile_asked &&
+    lc.padded = may_pad && max_vec >= 8 && lc.variant != GMR_VARIANT_PERSISTENT && !tile_asked &&
                 needs_padding(e, semiring, lc.Bw, aligned(16));
     if (lc.padded) {
         const int nt = (lc.Bw + 127) / 128, per = (lc.Bw + nt - 1) / nt;
@@ -1835,25 +1836,77 @@ static int64_t run_chain(gmr_engine* e, const Launch& lc, GraphEntry::Kind kind,
     return hit->launches;
 }
 
-// Grows the value arena and terminal table; cached graphs bake these
-// addresses in, so any reallocation drops them (after the device is idle).
-static void ensure_scratch(gmr_engine* e, int words, int64_t padx_rows = 0, int64_t pady_rows = 0) {
-    const size_t na = (size_t)std::max<int64_t>(e->n_ops, 1) * words * 4;
-    const size_t nt = (size_t)std::max<int64_t>(e->n_terms, 1) * words * 4;
-    const size_t ny = (size_t)pady_rows * words * 4, nx = (size_t)padx_rows * words * 4;
-    if (na <= e->arena.bytes && nt <= e->T.bytes && ny <= e->padY.bytes && nx <= e->padX.bytes) return;
+// Scratch of a product, in bytes: value arena, terminal table, padded X and Y.
+struct Scratch {
+    size_t arena, T, padX, padY;
+    Scratch(const gmr_engine* e, int words, int64_t padx_rows, int64_t pady_rows)
+        : arena((size_t)std::max<int64_t>(e->n_ops, 1) * words * 4),
+          T((size_t)std::max<int64_t>(e->n_terms, 1) * words * 4),
+          padX((size_t)padx_rows * words * 4),
+          padY((size_t)pady_rows * words * 4) {}
+    size_t total() const { return arena + T + padX + padY; }
+};
+static Scratch right_scratch(const gmr_engine* e, const Launch& lc) {
+    return {e, lc.Bp, lc.padded && e->direct_terms ? e->cols : 0, lc.padded ? e->rows : 0};
+}
+
+// Grows the scratch; cached graphs bake these addresses in, so any
+// reallocation drops them (after the device is idle).
+static void ensure_scratch(gmr_engine* e, const Scratch& n) {
+    if (n.arena <= e->arena.bytes && n.T <= e->T.bytes && n.padY <= e->padY.bytes && n.padX <= e->padX.bytes) return;
     GMR_CUDA(cudaDeviceSynchronize());
     for (auto& g : e->graphs)
         if (g.exec) cudaGraphExecDestroy(g.exec);
     e->graphs.clear();
-    e->arena.ensure(na);
-    e->T.ensure(nt);
-    e->padY.ensure(ny);
-    e->padX.ensure(nx);
+    e->arena.ensure(n.arena);
+    e->T.ensure(n.T);
+    e->padY.ensure(n.padY);
+    e->padX.ensure(n.padX);
 }
 
-static void ensure_scratch(gmr_engine* e, const Launch& lc) {  // of a right product
-    ensure_scratch(e, lc.Bp, lc.padded && e->direct_terms ? e->cols : 0, lc.padded ? e->rows : 0);
+// The launch that resolve(may_pad) gives, with its scratch (size(launch)) at hand.
+// What only makes a product faster goes when the device has no memory for it:
+// the padded layout (not tried again for as much), then the one-word lists.
+template <class R, class N>
+static Launch resolve_with_scratch(gmr_engine* e, R&& resolve, N&& size) {
+    auto fits = [&](const Launch& lc) {
+        try {
+            ensure_scratch(e, size(lc));
+            return true;
+        } catch (const Error& err) {
+            if (err.code != GMR_ERR_OOM) throw;
+            return false;
+        }
+    };
+    Launch lc = resolve(true);
+    if (lc.padded) {
+        const size_t need = size(lc).total();
+        if (need < e->pad_refused) {
+            if (fits(lc)) return lc;
+            e->pad_refused = need;
+            e->padX.release();  // the device is idle and no graph is left (ensure_scratch)
+            e->padY.release();
+        }
+        lc = resolve(false);
+    }
+    const bool lists = e->word.ready || e->left_word.ready;
+    if (lists && !fits(lc)) {
+        e->word.ready = e->left_word.ready = false;
+        for (auto* b : {&e->word.entries, &e->word.seg, &e->word_parts, &e->left_word.entries, &e->left_word.seg,
+                        &e->lp_src, &e->lp_tgt})
+            b->release();
+        lc = resolve(false);
+    }
+    ensure_scratch(e, size(lc));
+    return lc;
+}
+
+// resolve_launch with the scratch of a right product.
+static Launch resolve_right(gmr_engine* e, int semiring, int B, const void* X, void* Y, const gmr_config* cfg,
+                            int max_vec = 8) {
+    return resolve_with_scratch(
+        e, [&](bool may_pad) { return resolve_launch(e, semiring, B, X, Y, cfg, max_vec, may_pad); },
+        [&](const Launch& lc) { return right_scratch(e, lc); });
 }
 
 static void multiply_device(gmr_engine* e, int semiring, const void* X, void* Y, int B, const gmr_config* cfg,
@@ -1862,9 +1915,8 @@ static void multiply_device(gmr_engine* e, int semiring, const void* X, void* Y,
     if (B < 1) throw Error(GMR_ERR_ARG, "B must be >= 1");
     if ((!X && e->cols > 0) || (!Y && e->rows > 0)) throw Error(GMR_ERR_ARG, "null X or Y");
     if (((uintptr_t)X | (uintptr_t)Y) % 4 != 0) throw Error(GMR_ERR_ARG, "X and Y must be 4-byte aligned");
-    Launch lc = resolve_launch(e, semiring, B, X, Y, cfg);
+    Launch lc = resolve_right(e, semiring, B, X, Y, cfg);
     if (eager && lc.variant == GMR_VARIANT_GRAPH) lc.variant = GMR_VARIANT_FUSED;
-    ensure_scratch(e, lc);
     int64_t launches = 0;
     if (lc.variant == GMR_VARIANT_GRAPH) {
         launches = run_chain(e, lc, GraphEntry::kRight, X, Y, st,
@@ -2919,17 +2971,17 @@ static void left_chain_s(gmr_engine* e, const Launch& lc, const void* X, void* Y
 }
 
 // Widths and lanes of a left product: the right product's rules, one tile.
-static Launch resolve_left(gmr_engine* e, int semiring, int B, const void* X, void* Y) {
+static Launch resolve_left(gmr_engine* e, int semiring, int B, const void* X, void* Y, bool may_pad) {
     Launch lc{};
     lc.semiring = semiring;
     lc.B = B;
     lc.Bw = words_per_slot(semiring, B);
     auto aligned = [&](size_t al) { return ((uintptr_t)X % al == 0) && ((uintptr_t)Y % al == 0); };
-    lc.padded = needs_padding(e, semiring, lc.Bw, aligned(16));
+    lc.padded = may_pad && needs_padding(e, semiring, lc.Bw, aligned(16));
     lc.Bt = lc.Bp = lc.padded ? padded_words(lc.Bw) : lc.Bw;
     lc.ntile = 1;
     if (semiring == GMR_PLUS_TIMES && lc.Bp % 8 == 0 && lc.Bp >= 32 && (lc.padded || aligned(32))) lc.VEC = 8;
-    else if (lc.Bp % 4 == 0) lc.VEC = 4;  // not padded: 16-byte aligned
+    else if (lc.Bp % 4 == 0 && (lc.padded || aligned(16))) lc.VEC = 4;
     else if (lc.Bp == 2 && aligned(8)) lc.VEC = 2;
     else lc.VEC = 1;
     lc.G = lc.Bp / lc.VEC;
@@ -3045,8 +3097,9 @@ extern "C" int gmr_engine_multiply_left(gmr_engine* e, int semiring, const void*
         if (((uintptr_t)dX | (uintptr_t)dY) % 4 != 0) throw Error(GMR_ERR_ARG, "X and Y must be 4-byte aligned");
         std::lock_guard<std::mutex> lk(e->mu);
         DeviceGuard dg(e->device);
-        const Launch lc = resolve_left(e, semiring, B, dX, dY);
-        ensure_scratch(e, lc.Bp, lc.padded ? e->rows : 0, lc.padded ? e->cols : 0);
+        const Launch lc = resolve_with_scratch(
+            e, [&](bool may_pad) { return resolve_left(e, semiring, B, dX, dY, may_pad); },
+            [&](const Launch& l) { return Scratch(e, l.Bp, l.padded ? e->rows : 0, l.padded ? e->cols : 0); });
         e->last_launches = run_chain(e, lc, GraphEntry::kLeft, dX, dY, static_cast<cudaStream_t>(stream),
                                      [&](cudaStream_t st, int64_t& n) {
                                          if (semiring == GMR_PLUS_TIMES) left_chain_s<SPlus>(e, lc, dX, dY, st, n);
@@ -3173,9 +3226,8 @@ extern "C" int gmr_engine_fixpoint(gmr_engine* e, int semiring, void* dX, void* 
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         if (iters) *iters = 0;
         if (max_iters == 0) return;
-        Launch lc = resolve_launch(e, semiring, B, dX, dY, nullptr);
+        Launch lc = resolve_right(e, semiring, B, dX, dY, nullptr);
         if (lc.variant == GMR_VARIANT_GRAPH || lc.variant == GMR_VARIANT_PERSISTENT) lc.variant = GMR_VARIANT_FUSED;
-        ensure_scratch(e, lc);
         const int64_t n = (int64_t)e->rows * lc.Bw;
         e->sync.ensure(64);
         int* flag = reinterpret_cast<int*>(static_cast<unsigned char*>(e->sync.p) + 8);
@@ -3471,9 +3523,7 @@ extern "C" int gmr_pack_multiply(gmr_pack* p, const int* semirings, const void* 
             if (semirings[i] < 0 || semirings[i] > 2) throw Error(GMR_ERR_ARG, "unknown semiring");
             if (B[i] < 1) throw Error(GMR_ERR_ARG, "B must be >= 1");
             if (((uintptr_t)dX[i] | (uintptr_t)dY[i]) % 4 != 0) throw Error(GMR_ERR_ARG, "misaligned X or Y");
-            Launch lc = resolve_launch(e, semirings[i], B[i], dX[i], dY[i], nullptr, one_kernel ? 4 : 8);
-            ensure_scratch(e, lc);
-            lcs.push_back(lc);
+            lcs.push_back(resolve_right(e, semirings[i], B[i], dX[i], dY[i], nullptr, one_kernel ? 4 : 8));
         }
         p->last_persistent = false;
         if (p->mode == GMR_PACK_PERSISTENT && uniform && !direct) {
