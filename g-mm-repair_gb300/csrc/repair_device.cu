@@ -242,11 +242,11 @@ T read1(const T* d, cudaStream_t st) {
         GMR_CUDA(cudaGetLastError());                                   \
     } while (0)
 
-// At least n elements, with room to spare when it has to grow (its contents
-// are not kept).
+// At least n elements (contents are not kept), and no more when it has to grow: the
+// round with the most pairs needs what it needed with buffers of its own.
 template <class T>
 void reserve(DevArray<T>& a, int64_t n) {
-    if (a.n < n || !a.p) a.alloc(n + n / 4 + 1);
+    if (a.n < n || !a.p) a.alloc(n);
 }
 
 struct Stream {
