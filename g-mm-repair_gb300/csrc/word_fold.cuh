@@ -10,8 +10,8 @@
 // order, 4 bytes each: the source's place in the chunk and the row's in its
 // block of 65,536 rows, 16 bits each (half the 8 bytes of the level order).
 // Each block takes an equal share of that list, loads the few chunks it spans
-// with coalesced reads and reduces every row's run in registers; each run is
-// one reduction into Y.
+// with coalesced reads and reduces every row's run in registers, a warp 128
+// emissions at a time; each run within those 128 is one reduction into Y.
 //
 // With the gathers out of the way the instruction rate bounds it: a first form
 // with one emission per lane and a shuffle scan over the 32 rows of every warp
@@ -44,8 +44,13 @@ constexpr int64_t kWordMinEmissions = 1 << 16, kWordMinEmissionsPlus = 2 << 20;
 // The left product pays two launches for it, about 10 us, and saves 26 us at
 // 15 M emissions (50,000 x 5,000); at 0.5 M (1,479 x 2,064) it lost 27 -> 37 us.
 constexpr int64_t kLeftWordMinEmissions = 6 << 20;
-// Chunks per copy of Y: a row gets one addition per chunk that emits into it,
-// and the error of that chain grows with its length.
+// Chunks per copy of Y: a row gets an addition per chunk that emits into it, more
+// where its run there is longer than a warp step (n / 128 + 1 for n emissions),
+// and the error of that chain grows with its length.  Long runs shorten it: the
+// per-level fold they replace adds once per 32 to 128 emissions too, in every
+// level.  Error against 64 bits, worst row over the largest value, per-level
+// default before -> one launch: 41 rows x 400,000 (2.2 M emissions) 3.2e-6 ->
+// 2.5e-6, 8 x 2,000,000 (2.6 M) 1.8e-6 -> 0.9e-6.
 constexpr int kWordChunksPerCopy = 16, kWordMaxCopies = 16;
 
 // Where the arena starts in the value space: a whole number of 256-byte lines.
