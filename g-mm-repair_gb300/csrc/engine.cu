@@ -3066,17 +3066,7 @@ extern "C" int gmr_engine_enable_left(gmr_engine* e, gmr_plan* p) {
             upload(tgt, e->lp_tgt);
         }
         // targets whose edges straddle the chunks used here (the plan's list is for kLeftChunk throughout)
-        std::vector<int32_t> split;
-        for (int k = 1; k <= e->depth + 1; ++k) {
-            const int64_t lo = p->le_off[k - 1], hi = p->le_off[k], c = left_chunk(hi - lo);
-            int32_t before = -1;
-            for (int64_t b = lo + c; b < hi; b += c) {  // chunk boundaries: the target on both sides
-                const int32_t t = p->le_tgt[b];
-                if (t != p->le_tgt[b - 1] || t == before) continue;
-                split.push_back(k <= e->depth ? t : (int32_t)(e->n_ops + t));
-                before = t;
-            }
-        }
+        const std::vector<int32_t> split = left_split(p->le_off, p->le_tgt, e->n_ops, left_chunk);
         upload(split, e->le_split);
         upload(p->tcol_off, e->tcol_off);
         upload(p->tcol_q, e->tcol_q);

@@ -113,7 +113,24 @@ struct gmr_plan {
 };
 
 namespace gmr {
-constexpr int64_t kLeftChunk = 16;  // edges per lane group in the left fold
+constexpr int64_t kLeftChunk = 16;  // edges per chunk of a plan's le_split
+// The targets (le_split's encoding) whose edges straddle a chunk, with
+// chunk_of(n) edges per chunk in a range of n: those on both sides of a boundary.
+template <class F>
+std::vector<int32_t> left_split(const std::vector<int64_t>& off, const std::vector<int32_t>& tgt, int64_t n_ops, F&& chunk_of) {
+    std::vector<int32_t> split;
+    for (size_t k = 1; k < off.size(); ++k) {
+        const int64_t lo = off[k - 1], hi = off[k], c = chunk_of(hi - lo);
+        int32_t before = -1;
+        for (int64_t b = lo + c; b < hi; b += c) {
+            const int32_t t = tgt[b];
+            if (t != tgt[b - 1] || t == before) continue;
+            split.push_back(k + 1 < off.size() ? t : (int32_t)(n_ops + t));
+            before = t;
+        }
+    }
+    return split;
+}
 void validate_plan(const gmr_plan& p);  // throws Error(GMR_ERR_FORMAT)
 void fill_common_stats(gmr_plan& p);    // stats derived from the plan arrays
 // Lanes per value of a multiply of (semiring, B), 0 where the engine folds all

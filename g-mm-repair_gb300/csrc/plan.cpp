@@ -682,17 +682,7 @@ extern "C" int gmr_plan_prepare_left(gmr_plan* p) {
         std::vector<int64_t> lo((size_t)D + 2, 0);
         for (int k = 1; k <= D; ++k) lo[k] = p->lvl_off[k] < n ? start[p->lvl_off[k]] : (po[n] - po[0]) + (eo[n] - eo[0]);
         lo[D + 1] = tot;
-        std::vector<int32_t> split;
-        for (int k = 1; k <= D + 1; ++k) {
-            const int64_t a = lo[k - 1], b = lo[k];
-            for (int64_t e = a; e < b;) {
-                int64_t f = e + 1;
-                while (f < b && tgt[f] == tgt[e]) ++f;
-                if ((e - a) / kLeftChunk != (f - 1 - a) / kLeftChunk)
-                    split.push_back(k <= D ? tgt[e] : (int32_t)(n + tgt[e]));
-                e = f;
-            }
-        }
+        std::vector<int32_t> split = left_split(lo, tgt, n, [](int64_t) { return kLeftChunk; });
         p->par_off.swap(po);
         p->erow_off.swap(eo);
         p->tcol_off.swap(co);
