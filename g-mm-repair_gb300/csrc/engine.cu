@@ -513,7 +513,12 @@ __device__ __forceinline__ void do_emits_atomic(const SweepArgs& a, const LevelA
 // on those: a step of 32 frontiers on 8 M nodes 1090 -> 691 us, a (min,+) step
 // on 2 M nodes 307 -> 212 us.  Levels whose emissions fit the GPU's lanes at once
 // (em_chunk = 1) keep one per lane, with twice the warps and a shorter chain:
-// 2,000 x 1,000, (+,x) 34.2 us with four per lane throughout, 29.4 with one.
+// 2,000 x 1,000, (+,x) 34.2 us with four per lane throughout, 29.4 with one.  The
+// line at 2,048 emissions per SM, one for each of its lanes, is the same for all
+// semirings (20,000 x 5,000, level by level, at 1,024 / 2,048 / 4,096 / 8,192:
+// (+,x) B = 1 71.7 / 68.9 / 69.9 / 73.1 us, B = 4 88.0 / 86.0 / 88.4 / 94.6; 128
+// Boolean columns 90.5 / 88.3 / 91.8 / 99.3; 6,000 x 2,000, (+,x) B = 1 42.9 / 41.0 /
+// 41.0 / 41.0; 98,160 x 7,210 within 1 %).
 template <class S, int VEC, bool CG = false, bool DIR = false>
 __device__ __forceinline__ void do_emits_warp(const SweepArgs& a, const LevelArgs& L, int tile, const Span& sp) {
     using T = typename S::T;
@@ -1388,7 +1393,7 @@ static void launch_chain_t(gmr_engine* e, const Launch& lc, const void* X, void*
         // fit the GPU at once.
         auto chunk_of = [&](int64_t ne, int c) {
             if constexpr (GLOG == 0) {
-                return ne <= (int64_t)e->sm_count * (std::is_same<S, SPlus>::value ? 8192 : 2048) ? 1 : 4;  // per lane
+                return ne <= (int64_t)e->sm_count * 2048 ? 1 : 4;  // per lane
             } else {
                 while (c > 4 && (ne + c / 2 - 1) / (c / 2) * lc.G <= (int64_t)e->sm_count * 1024) c /= 2;
                 return (c + 3) & ~3;
