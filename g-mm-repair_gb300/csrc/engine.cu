@@ -2897,7 +2897,7 @@ static void left_chain_t(gmr_engine* e, const Launch& lc, const void* X, void* Y
         ++launches;
     };
     const int D = e->depth;
-    if constexpr (VEC == 1 && GLOG == 0) {
+    if constexpr (VEC == 1 && GLOG == 0 && std::is_same<S, SPlus>::value) {
         if (lc.word) {  // all rows' parts in one launch out of shared memory, then the parents level by level
             a.count = e->n_terms;
             launch(k_left_clear<S>, blocks(e->n_ops + e->n_terms), a);
@@ -2995,7 +2995,7 @@ static Launch resolve_left(gmr_engine* e, int semiring, int B, const void* X, vo
     else if (lc.Bp == 2 && aligned(8)) lc.VEC = 2;
     else lc.VEC = 1;
     lc.G = lc.Bp / lc.VEC;
-    lc.word = lc.Bw == 1 && e->left_word.ready && aligned(16);
+    lc.word = semiring == GMR_PLUS_TIMES && lc.Bw == 1 && e->left_word.ready && aligned(16);
     return lc;
 }
 

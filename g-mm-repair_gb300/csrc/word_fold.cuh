@@ -41,9 +41,15 @@ constexpr int kWordGroup = 128;     // emissions per warp step: four per lane
 // 119 -> 64).
 constexpr double kWordMinPerRow = 0.25;
 constexpr int64_t kWordMinEmissions = 1 << 16, kWordMinEmissionsPlus = 2 << 20;
-// The left product pays two launches for it, about 10 us, and saves 26 us at
-// 15 M emissions (50,000 x 5,000); at 0.5 M (1,479 x 2,064) it lost 27 -> 37 us.
-constexpr int64_t kLeftWordMinEmissions = 6 << 20;
+// The left product, (+,x) only: two launches more, and every down value is read
+// and written once more.  One product, edge lists alone -> rows' edges at once:
+// 20,000 x 5,000 (6.5 M emissions) 100 -> 115 us, 80,001 x 1,500 (7.0 M) 101 -> 117,
+// 25,000 x 5,000 (8.0 M) 118 -> 123, 30,000 x 5,000 (9.6 M) 120 -> 117, 35,000 x 5,000
+// (11.0 M) 139 -> 126, 160,001 x 1,500 (13.1 M) 146 -> 141, 50,000 x 5,000 (15.3 M)
+// 164 -> 155, 98,160 x 7,210 (40.7 M) 295 -> 245, 200,000 x 10,000 (109 M) 664 -> 647.
+// The idempotent semirings, whose atomics on down values are slower, lose on most:
+// (OR,AND) 11.0 M 129 -> 123, 15.3 M 151 -> 173, 40.7 M 279 -> 290, 109 M 627 -> 703.
+constexpr int64_t kLeftWordMinEmissions = 9 << 20;
 // Chunks per copy of Y: a row gets an addition per chunk that emits into it, more
 // where its run there is longer than a warp step (n / 128 + 1 for n emissions),
 // and the error of that chain grows with its length.  Long runs shorten it: the

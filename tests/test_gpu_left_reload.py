@@ -32,8 +32,8 @@ def small():
 
 
 @pytest.fixture(scope="module")
-def large():  # above the 6 Mi emissions from which one-word products fold the rows' edges at once
-    return _plans(80001, 1500, 64) + (80001, 1500)
+def large():  # above the 9 Mi emissions from which one-word (+,x) products fold the rows' edges at once
+    return _plans(120001, 1500, 64) + (120001, 1500)
 
 
 @pytest.mark.parametrize("size", ["small", "large"])

@@ -96,7 +96,7 @@ def test_left_list(sr):
     """Rows beyond one chunk of x, targets in several blocks of 65,536; an x off
     the 16-byte boundary takes the edge lists."""
     torch = pytest.importorskip("torch")
-    d = _build(gmr.gen_mosaic(80001, 1500, 64, 0.01, 1e-3, 3))
+    d = _build(gmr.gen_mosaic(120001, 1500, 64, 0.01, 1e-3, 3))
     assert int(d["plan"].array("em_off")[-1]) >= _constant("kLeftWordMinEmissions") and d["rows"] > CHUNK
     eng = gmr.Engine(d["plan"])
     before = eng.device_bytes
