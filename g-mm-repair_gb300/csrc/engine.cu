@@ -2133,14 +2133,14 @@ static void build_push_lists(const gmr_plan& p, gmr_engine& e) {
 // the GPU: of `values` values into `targets` targets, the left product's when
 // left_terms >= 0 (its terminals' first target).  emissions() gives the device
 // arrays; it is called once it is known that the list pays.  Not built where
-// it does not pay: graphs with direct terminals (their terminals are no table),
-// too few emissions, runs too short (kWordMinPerRow).
+// it does not pay (kWordMinDepth and on), nor for graphs with direct terminals
+// (their terminals are no table).
 template <class F>
 static void build_word_list(gmr_engine& e, WordList& l, F&& emissions, int64_t E, int64_t values, int64_t targets,
-                            int64_t left_terms, int64_t min_emissions) {
+                            int64_t left_terms, int64_t min_emissions, double min_per_target) {
     const int64_t chunks = (values + kWordChunk - 1) / kWordChunk, blks = (targets + 65535) / 65536;
-    if (e.direct_terms || e.n_ops == 0 || E < min_emissions || E >= (int64_t)UINT32_MAX - 1 ||
-        (double)E < kWordMinPerRow * (double)chunks * (double)targets || chunks * blks > (1 << 20))
+    if (e.direct_terms || e.n_ops == 0 || e.depth < kWordMinDepth || E < min_emissions || E >= (int64_t)UINT32_MAX - 1 ||
+        (double)E < min_per_target * (double)chunks * (double)targets || chunks * blks > (1 << 20))
         return;
     const int row_bits = std::max(16, bits_for((uint64_t)targets));  // at least the 16 bits an entry keeps
     const int n_seg = (int)(chunks * blks);
@@ -2184,7 +2184,7 @@ static void build_word_fold(gmr_engine& e) {
     auto emissions = [&] {
         return std::pair(static_cast<const int32_t*>(e.em_src.p), static_cast<const int32_t*>(e.em_row.p));
     };
-    build_word_list(e, e.word, emissions, e.n_em, values, e.rows, -1, kWordMinEmissions);
+    build_word_list(e, e.word, emissions, e.n_em, values, e.rows, -1, kWordMinEmissions, kWordMinPerRow);
     e.word_copies = (int)std::min<int64_t>(kWordMaxCopies, (chunks + kWordChunksPerCopy - 1) / kWordChunksPerCopy);
     if (!e.word.ready || e.word_copies == 1) return;
     if (!build_order([&] { e.word_parts.ensure((size_t)e.rows * e.word_copies * 4); })) e.word_copies = 1;
@@ -3054,7 +3054,8 @@ extern "C" int gmr_engine_enable_left(gmr_engine* e, gmr_plan* p) {
                 return std::pair<const int32_t*, const int32_t*>(upload(p->em_src, src), upload(p->em_row, row));
             };
             build_word_list(*e, e->left_word, emissions, (int64_t)p->em_src.size(), e->rows,
-                            left_word_terms(e) + e->n_terms, left_word_terms(e), kLeftWordMinEmissions);
+                            left_word_terms(e) + e->n_terms, left_word_terms(e), kLeftWordMinEmissions,
+                            kLeftWordMinPerTarget);
         }
         if (e->left_word.ready) {
             const int D = e->depth;

@@ -30,26 +30,48 @@ namespace gmr {
 constexpr int kWordChunk = 57344;   // words of values per chunk: 224 KB of a block's 227 KB, and 16-bit places
 constexpr int kWordThreads = 1024;  // one block per SM
 constexpr int kWordGroup = 128;     // emissions per warp step: four per lane
-// Where the fold pays (one multiply as a graph, per-level folds -> this one).
-// Emissions per chunk and row: long enough runs; a chunk of a mosaic holds 1
-// to 60 emissions per row, graphs below 0.25 were not measured faster.
-// Emissions in all: (+,x) loses below about 2 M (5,000 x 2,000, 1.4 M: 40.8 ->
-// 43.4 us) and gains above (100,000 x 600, 3 M: 55.6 -> 50.7; 20,000 x 5,000,
-// 6.6 M: 76 -> 64; 200,000 x 10,000, 109 M: 625 -> 322); the idempotent
-// semirings, whose per-level fold reduces run by run, gain from the start
-// (20,000 nodes of degree 24, (OR,AND): 47 -> 25; 20,000 x 5,000, (min,+):
-// 119 -> 64).
+// Where the fold pays (one multiply as a graph, level by level -> in one launch).
+// It takes the emissions off every level's launch and pays a launch and the loads
+// of the chunks for it, so the levels have to be many: grammars of mosaics have 14
+// to 23, of copy graphs 6 to 13.  Right product:
+//   mosaics          levels  emissions  per chunk and row   (+,x) us      (OR,AND) us
+//   1,500 x 800        19      0.10 M      67                -            36.9 ->  34.8
+//   5,000 x 2,000      20      0.75 M      50                -            44.1 ->  45.0
+//   9,000 x 3,000      21      1.9 M       30                -            53.3 ->  49.3
+//   40,000 x 1,000     19      2.5 M        7.7          47.2 ->  47.8    52.6 ->  47.1
+//   20,000 x 5,000     23      6.5 M       15            69.6 ->  65.2    74.1 ->  62.6
+//   600,000 x 300      17      8.9 M        0.67         75.8 ->  72.7    79.9 ->  67.0
+//   1,500,000 x 150    14     10.4 M        0.30         84.1 ->  87.2    87.8 ->  77.9
+//   400,000 x 1,000     -     20.6 M        0.99        139.7 -> 113.9   144.4 -> 109.2
+//   98,160 x 7,210      -     40.7 M        3.6         239.5 -> 151.8   240.2 -> 146.1
+//   200,000 x 10,000    -    109 M          1.9           625 -> 322         -
+//   copy graphs (nodes, degree, share copied)
+//   20,000, 48, 0.7     7      0.54 M       9.0              -            20.5 ->  26.6
+//   200,000, 16, 0.8    9      1.4 M        0.58             -            32.7 ->  36.9
+//   100,000, 48, 0.5    6      3.7 M        3.7          30.6 ->  32.8    32.8 ->  32.8
+//   300,000, 32, 0.8   11      4.2 M        0.47         51.0 ->  57.4    53.3 ->  55.1
+//   500,000, 24, 0.6    7      8.1 M        0.48         63.2 ->  71.9    65.6 ->  67.5
+//   200,000, 100, 0.7   9     11.4 M        1.09         82.8 ->  82.2    85.2 ->  77.8
+//   300,000, 100, 0.7   9     17.1 M        0.74        113.1 -> 123.0   115.4 -> 117.6
+// (min,+) is within 3 % of (OR,AND).  (+,x) lost below 2 M (a mosaic of 1.4 M: 40.8
+// -> 43.4), and is within 1 % from there to 4 M.  Below 0.25 per chunk and row not
+// measured.
+constexpr int kWordMinDepth = 14;
 constexpr double kWordMinPerRow = 0.25;
 constexpr int64_t kWordMinEmissions = 1 << 16, kWordMinEmissionsPlus = 2 << 20;
 // The left product, (+,x) only: two launches more, and every down value is read
-// and written once more.  One product, edge lists alone -> rows' edges at once:
-// 20,000 x 5,000 (6.5 M emissions) 100 -> 115 us, 80,001 x 1,500 (7.0 M) 101 -> 117,
-// 25,000 x 5,000 (8.0 M) 118 -> 123, 30,000 x 5,000 (9.6 M) 120 -> 117, 35,000 x 5,000
-// (11.0 M) 139 -> 126, 160,001 x 1,500 (13.1 M) 146 -> 141, 50,000 x 5,000 (15.3 M)
-// 164 -> 155, 98,160 x 7,210 (40.7 M) 295 -> 245, 200,000 x 10,000 (109 M) 664 -> 647.
+// and written once more.  The same depth, and emissions per chunk of x and target
+// (rules and terminals).  One product, edge lists alone -> rows' edges at once:
+//   20,000 x 5,000     6.5 M  4.7  100 -> 115 us    50,000 x 5,000    15.3 M  5.6  164 -> 155
+//   80,001 x 1,500     7.0 M  2.7  101 -> 117       100,000 x 4,000   22.9 M  2.9  207 -> 185
+//   25,000 x 5,000     8.0 M  5.0  118 -> 123       98,160 x 7,210    40.7 M  3.1  295 -> 245
+//   30,000 x 5,000     9.6 M  5.4  120 -> 117       200,000 x 10,000  109 M   1.6  664 -> 647
+//   35,000 x 5,000    11.0 M  5.5  139 -> 126       1,500,000 x 150   10.4 M  0.3  111 -> 144
+//   160,001 x 1,500   13.1 M  1.9  146 -> 141       graph 300,000 x 100  17 M  0.7  143 -> 197
 // The idempotent semirings, whose atomics on down values are slower, lose on most:
 // (OR,AND) 11.0 M 129 -> 123, 15.3 M 151 -> 173, 40.7 M 279 -> 290, 109 M 627 -> 703.
 constexpr int64_t kLeftWordMinEmissions = 9 << 20;
+constexpr double kLeftWordMinPerTarget = 1.5;
 // Chunks per copy of Y: a row gets an addition per chunk that emits into it, more
 // where its run there is longer than a warp step (n / 128 + 1 for n emissions),
 // and the error of that chain grows with its length.  Long runs shorten it: the

@@ -1,6 +1,7 @@
 """The one-launch fold of 4-byte values where its other tests do not take it:
-several copies of Y, (+,x) on long rows and graphs above its threshold, the left
-product's list, packs, the timing recorder and the autotuner.  Each case states
+several copies of Y, (+,x) on long and on short rows above its threshold, a list of
+one chunk, the left product's list, packs, the fixpoint loop, the timing recorder
+and the autotuner.  Each case states
 from the plan that the fold applies.  (+,x) within 1e-5 relative max-norm of
 FP64, the others exact."""
 import re
@@ -30,9 +31,10 @@ def _chunks(plan):
     return -(-((plan.stats["n_terms"] + 63) // 64 * 64 + plan.stats["n_ops"]) // CHUNK)
 
 
-def _folds_plus(plan, rows):
+def _folds(plan, rows, least):
     E = int(plan.array("em_off")[-1])
-    return E >= _constant("kWordMinEmissionsPlus") and E >= _constant("kWordMinPerRow") * _chunks(plan) * rows
+    return (E >= _constant(least) and E >= _constant("kWordMinPerRow") * _chunks(plan) * rows
+            and plan.stats["depth"] >= _constant("kWordMinDepth"))
 
 
 def _build(m):
@@ -46,21 +48,21 @@ def _build(m):
 @pytest.fixture(scope="module")
 def copies():  # 19 chunks: two copies of Y
     d = _build(gmr.gen_mosaic(70001, 1500, 64, 0.01, 1e-3, 3))
-    assert _chunks(d["plan"]) > PER_COPY and _folds_plus(d["plan"], d["rows"])
+    assert _chunks(d["plan"]) > PER_COPY and _folds(d["plan"], d["rows"], "kWordMinEmissionsPlus")
     return d
 
 
 CASES = {
     "copies": None,
     "long_rows": lambda: gmr.gen_mosaic(41, 400000, 16, 0.02, 0.01, 4),
-    "graph": lambda: gmr.gen_copy_graph(300000, 24, 0.7, False, 5),
+    "short_rows": lambda: gmr.gen_mosaic(300000, 300, 64, 0.01, 1e-3, 0),
 }
 
 
 @pytest.mark.parametrize("name", list(CASES))
 def test_plus_times_above_its_threshold(name, request):
     d = request.getfixturevalue("copies") if CASES[name] is None else _build(CASES[name]())
-    assert _folds_plus(d["plan"], d["rows"])
+    assert _folds(d["plan"], d["rows"], "kWordMinEmissionsPlus")
     eng = gmr.Engine(d["plan"])
     x = np.random.default_rng(7).uniform(-1, 1, d["cols"]).astype(np.float32)
     ref = np.bincount(d["r"], d["v"] * x[d["c"]].astype(np.float64), d["rows"])
@@ -133,9 +135,9 @@ def test_left_list(sr):
 def test_pack_of_one_word_engines(copies):
     """Branches of a pack's graph with the fold, two copies of Y in one of them."""
     torch = pytest.importorskip("torch")
-    g = _build(gmr.gen_copy_graph(21000, 12, 0.7, False, 5))
+    g = _build(gmr.gen_mosaic(1500, 800, 64, 0.01, 1e-3, 0))
     engs = [gmr.Engine(copies["plan"]), gmr.Engine(g["plan"])]
-    assert int(g["plan"].array("em_off")[-1]) >= _constant("kWordMinEmissions")
+    assert _folds(g["plan"], 1500, "kWordMinEmissions") and _chunks(g["plan"]) == 1
     rng = np.random.default_rng(3)
     X = [rng.uniform(-1, 1, (copies["cols"], 1)).astype(np.float32),
          rng.integers(0, 2**32, (g["cols"], 1), dtype=np.uint64).astype(np.uint32)]
@@ -181,3 +183,39 @@ def test_fixpoint_of_padded_batches(sr, words):
         dY = torch.empty_like(dX)
         assert eng.fixpoint_device(sr, dX.data_ptr(), dY.data_ptr(), B) == steps
         check(sr, engine_outputs(sr, dX.cpu().numpy().view(np.uint32 if sr == 1 else np.int32), B), ref)
+
+
+@pytest.fixture(scope="module")
+def square():
+    d = _build(gmr.gen_mosaic(1500, 1500, 64, 0.01, 1e-3, 0))
+    assert _folds(d["plan"], 1500, "kWordMinEmissions")
+    return d
+
+
+@pytest.mark.parametrize("sr,B", [(1, 1), (1, 32), (2, 1)])
+def test_few_chunks_and_the_fixpoint_loop(square, sr, B):
+    """Idempotent semirings fold in one launch from few emissions on: one product
+    and the loop's result against the per-level folds iterated from the host."""
+    torch = pytest.importorskip("torch")
+    n = square["rows"]
+    eng = gmr.Engine(square["plan"])
+    rng = np.random.default_rng(B)
+    if sr == 1:
+        x = np.zeros((n, 1), dtype=np.uint32)
+        x[rng.choice(n, B, replace=False), 0] = np.uint32(1) << np.arange(B, dtype=np.uint32)
+    else:
+        x = np.full((n, 1), 10**9, dtype=np.int32)
+        x[rng.choice(n, 3, replace=False)] = 0
+    dX = torch.from_numpy(x.view(np.int32).copy()).cuda()
+    dY = torch.empty_like(dX)
+    np.testing.assert_array_equal(eng.multiply(x, sr, B=B), eng.multiply(x, sr, B=B, push=gmr.PUSH_NEVER))
+    steps, ref = 0, x
+    while True:
+        y = eng.multiply(ref, sr, B=B, push=gmr.PUSH_NEVER)
+        new = ref | y if sr == 1 else np.minimum(ref, y)
+        steps += 1
+        if np.array_equal(new, ref):
+            break
+        ref = new
+    assert eng.fixpoint_device(sr, dX.data_ptr(), dY.data_ptr(), B) == steps
+    np.testing.assert_array_equal(dX.cpu().numpy().view(x.dtype), ref)
