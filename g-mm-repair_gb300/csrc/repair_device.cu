@@ -242,11 +242,15 @@ T read1(const T* d, cudaStream_t st) {
         GMR_CUDA(cudaGetLastError());                                   \
     } while (0)
 
-// At least n elements (contents are not kept), and no more when it has to grow: the
-// round with the most pairs needs what it needed with buffers of its own.
+// At least n elements (contents are not kept).  When it has to grow, with room to
+// spare as long as the device has plenty, else no more than a round's own buffer
+// would take.
 template <class T>
 void reserve(DevArray<T>& a, int64_t n) {
-    if (a.n < n || !a.p) a.alloc(n);
+    if (a.n >= n && a.p) return;
+    size_t free_bytes = 0, total = 0;
+    GMR_CUDA(cudaMemGetInfo(&free_bytes, &total));
+    a.alloc((size_t)n * sizeof(T) < free_bytes / 64 ? n + n / 4 + 1 : n);
 }
 
 struct Stream {
