@@ -349,16 +349,20 @@ def check_all_columns(sched, V, sr, Xh, Yh, rows, cols, B, threads):
     return out
 
 
+KERNEL_SOURCES = [f"g-mm-repair_gb300/csrc/{f}" for f in (
+    "engine.cu", "device_util.cuh", "async_copy.cuh", "emission_orders.cuh", "sort.cuh", "word_fold.cuh",
+    "gmr_internal.h")] + ["include/gmr.h"]
+
+
 def source_hash(table: str = "") -> str:
     """Hash of the sources that make the sweep kernels: a traffic figure is
     only reported for the build it was measured on."""
     import hashlib
 
     h = hashlib.sha256()
-    files = ["g-mm-repair_gb300/csrc/engine.cu", "g-mm-repair_gb300/csrc/device_util.cuh",
-             "g-mm-repair_gb300/csrc/async_copy.cuh", "g-mm-repair_gb300/csrc/gmr_internal.h", "include/gmr.h"]
+    files = list(KERNEL_SOURCES)
     if table == "learned":  # the table the cost models pick
-        files.append("g-mm-repair_gb300/gmr/models/cost_model.gmrmlp")
+        files += ["g-mm-repair_gb300/csrc/learn.cu", "g-mm-repair_gb300/gmr/models/cost_model.gmrmlp"]
         if (REPO / "g-mm-repair_gb300/gmr/models/mode_model.gmrmlp").exists():
             files.append("g-mm-repair_gb300/gmr/models/mode_model.gmrmlp")
     for f in files:

@@ -56,3 +56,15 @@ def test_cusparse_generic_baseline_small():
     assert ran, out
     assert all(e < 1e-5 for e in out["spmm_rel_err_vs_torch"].values()), out
     assert any(isinstance(v, float) for v in out["spmv_vps"].values()), out
+
+
+def test_traffic_hash_covers_every_header_of_the_kernels():
+    import re
+
+    sys.path.insert(0, str(BENCH.parent))
+    import bench
+
+    engine = BENCH.parent / "g-mm-repair_gb300" / "csrc" / "engine.cu"
+    included = set(re.findall(r'#include "([^"]+)"', engine.read_text()))
+    hashed = {Path(f).name for f in bench.KERNEL_SOURCES}
+    assert included <= hashed and "engine.cu" in hashed
