@@ -20,8 +20,9 @@
 //     multiply is D + 2 launches instead of the reference's 2D + 4, each placed
 //     while the one before drains (programmatic dependent launch);
 //   * emissions are sorted by (row, source): each run of a row is reduced in
-//     registers and issues one atomic; with one 4-byte word per value all levels'
-//     emissions are folded at the end out of shared memory (word_fold.cuh);
+//     registers and issues one atomic; with one 4-byte word per value and levels
+//     enough all emissions are folded at the end out of shared memory
+//     (word_fold.cuh);
 //   * the launch chain is captured into a graph at its second use and replayed.
 #include <cuda_runtime.h>
 #include <dlfcn.h>
@@ -2653,11 +2654,11 @@ extern "C" void gmr_engine_free(gmr_engine* e) {
 // words per value a warp folds 128 consecutive edges (fold_runs) instead of
 // each lane walking 16 of its own.
 // The launches follow each other by programmatic dependent launch in a cached
-// graph.  At one word per value the rows' edges, three quarters of all, are
-// folded at once out of shared memory (k_word_fold with x as its values), and
-// only the parents' go level by level.
-// Measured on 50,000 x 5,000 (20 M edges), before -> now: B = 1 342 -> 173 us, 157
-// with the rows' edges at once, B = 32 698 -> 454 us; 3,149 x 575, B = 2 137 -> 57
+// graph.  For (+,x) at one word per value the rows' edges, three quarters of all,
+// are folded at once out of shared memory where that pays (kLeftWordMinEmissions:
+// k_word_fold with x as its values), and only the parents' go level by level.
+// Measured on 50,000 x 5,000 (20 M edges), before -> now: B = 1 342 -> 164 us, 155
+// with the rows' edges at once, B = 32 698 -> 432 us; 3,149 x 575, B = 2 137 -> 57
 // us; 29,229 x 2,388, B = 10 330 -> 220 us.
 namespace gmr {
 

@@ -286,7 +286,11 @@ enum {
 };
 
 int gmr_engine_create(const gmr_plan* p, int device, gmr_engine** out);
-/* dX, dY: device pointers (layouts above). stream: cudaStream_t or NULL. */
+/* dX, dY: device pointers (layouts above). stream: cudaStream_t or NULL.  On a
+ * stream that is being captured the launches become part of the caller's graph
+ * (after a call of the same batch width, which allocates the scratch).  Where the
+ * device has no memory for what only makes products faster (a padded copy of
+ * odd batches, the one-launch fold's list) they run without it. */
 int gmr_engine_multiply(gmr_engine* e, int semiring, const void* dX, void* dY,
                         int B, const gmr_config* cfg, void* stream);
 /* Host buffers: copies X in, multiplies, copies Y out, synchronous. */
@@ -449,7 +453,10 @@ int gmr_engine_status(const gmr_engine* e, int* failed, int* phase);
  * leaf(V, value) over its terminals.  x is [rows][words], y [cols][words]
  * (words = B, or ceil(B/32) for GMR_BOOLEAN).  gmr_plan_prepare_left builds
  * the reverse adjacency (parents per symbol, emitting rows per symbol,
- * terminals per column) on the host; gmr_engine_enable_left uploads it.
+ * terminals per column) on the host; gmr_engine_enable_left uploads it: of the
+ * engine's plan, or of one with as many rules, rows, columns and levels and no
+ * more terminals.  Called again it replaces what was there, once the device is
+ * idle.
  * The reference has no counterpart in its engine; mm-repair's CPU mat-vec
  * reports both Ax and xA. */
 int gmr_plan_prepare_left(gmr_plan* p);
