@@ -2721,11 +2721,10 @@ __global__ void __launch_bounds__(256) k_left_zero(LeftArgs a) {
     });
 }
 
-// Resident blocks: five for the idempotent semirings (50,000 x 5,000, 15 M edges'
-// emissions: (min,+) B = 32 464 us a product, 505 left alone; 96 Boolean columns
-// 239 and 256).  (+,x) is left alone: bounds make it spill (B = 32, four blocks
-// 462 us, three 439, left alone 439; B = 8, five 263, four 243, left alone 243;
-// 6,000 x 2,000, B = 8: 84, 72, 72).
+// Resident blocks: five for the idempotent semirings (50,000 x 5,000: (min,+) B = 32
+// 464 us a product, 505 without a bound; 96 Boolean columns 239 and 256).  (+,x) has
+// none, which would make it spill (B = 32: four blocks 462 us, three 439, no bound
+// 439; B = 8: five 263, four 243, no bound 243; 6,000 x 2,000, B = 8: 84, 72, 72).
 template <class S, int VEC, int GLOG>
 __global__ void __launch_bounds__(256, std::is_same<S, SPlus>::value ? 1 : 5) k_left_fold(LeftArgs a) {
     using T = typename S::T;

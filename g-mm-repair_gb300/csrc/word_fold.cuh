@@ -32,8 +32,8 @@ constexpr int kWordThreads = 1024;  // one block per SM
 constexpr int kWordGroup = 128;     // emissions per warp step: four per lane
 // Where the fold pays (one multiply as a graph, level by level -> in one launch).
 // It takes the emissions off every level's launch and pays a launch and the loads
-// of the chunks for it, so the levels have to be many: grammars of mosaics have 14
-// to 23, of copy graphs 6 to 13.  Right product:
+// of the chunks for it, so the levels have to be many: grammars of mosaics mostly
+// have 14 to 23, of copy graphs 6 to 13.  Right product:
 //   mosaics          levels  emissions  per chunk and row   (+,x) us      (OR,AND) us
 //   1,500 x 800        19      0.10 M      67                -            36.9 ->  34.8
 //   5,000 x 2,000      20      0.75 M      50                -            44.1 ->  45.0

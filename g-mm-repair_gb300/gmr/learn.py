@@ -130,7 +130,8 @@ class Mlp:
 
 
 def choose_learned(eng: Engine, plan: Plan, model: Mlp, semiring, B: int, mode_model: Mlp | None = None) -> np.ndarray:
-    """Installs the model's per-launch choice; returns its predictions [slots][variants] (log us).
+    """Installs the model's per-launch choice; returns its predictions [slots][variants]
+    (log us; +inf for variants that are never chosen at this lane layout).
     With mode_model (applied in its training domain, (+,x) at B >= 32), the
     levels it predicts faster interleaved get GMR_LEVEL_INTERLEAVE."""
     slots = plan.stats["depth"] + 2
